@@ -610,8 +610,8 @@ static int upload_mesh(asohf_ctx* c, const asohf_mesh* mh, DevMesh* d, DAlloc A 
 }
 
 // ------------------------------------------------------------ staging
-// The store in bin order as float4 (x, y, z, m) plus the species index, so
-// a patch reads its candidates as contiguous runs (one run per (y, z) row of
+// The store in bin order as float4 (x, y, z, m) plus the species index (in
+// the mass's place when all masses are equal), so a patch reads its candidates as contiguous runs (one run per (y, z) row of
 // bins).
 #define NA ASOHF_NAMRX
 #define ZH (NA / 2)
@@ -620,13 +620,18 @@ static int upload_mesh(asohf_ctx* c, const asohf_mesh* mh, DevMesh* d, DAlloc A 
 __global__ void k_bin_stage(const int32_t* __restrict__ idx, int64_t n, int64_t ndep, const float* __restrict__ x,
                             const float* __restrict__ y, const float* __restrict__ z, const float* __restrict__ m,
                             const float4* __restrict__ rows, const int64_t* __restrict__ esp_end,
-                            float4* __restrict__ P, uint8_t* __restrict__ S) {
+                            float4* __restrict__ P, uint8_t* __restrict__ S, int spec_in_w) {
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
     int p = idx[t];
-    P[t] = rows ? rows[2 * (int64_t)p] : make_float4(x[p], y[p], z[p], m[p]);
-    int s = 0;
-    while (S && s < ASOHF_N_ESP - 1 && (int64_t)p >= esp_end[s]) s++;
-    if (S) S[t] = (int64_t)p < ndep ? (uint8_t)s : (uint8_t)255;  // 255: not deposited
+    float4 v = rows ? rows[2 * (int64_t)p] : make_float4(x[p], y[p], z[p], m[p]);
+    if (esp_end) {
+      int s = 0;
+      while (s < ASOHF_N_ESP - 1 && (int64_t)p >= esp_end[s]) s++;
+      if ((int64_t)p >= ndep) s = 255;  // not deposited
+      if (spec_in_w) v.w = __int_as_float(s);
+      else S[t] = (uint8_t)s;
+    }
+    P[t] = v;
   }
 }
 
@@ -713,27 +718,20 @@ __global__ void k_base_stencil(const int32_t* __restrict__ cnt, int nx, Terms27 
 }
 
 // ------------------------------------------------------------ patch deposit
-// Work unit: PZ z-planes of one patch, accumulated in float64 shared memory.
-// A unit's candidates are the particles of the bins that overlap the patch
-// box extended by MAXKERNELEXT = DX (grids.f:837-893), restricted in z to
-// the unit's planes +- DX; they are split into slices of PSLICE so that a
-// dense unit is shared by several CTAs, whose sums meet in a float64 scratch
-// slab.  Inside a CTA all warps stride over the unit's candidates as one
-// flat range.  A hit whose kernel level is 0 (27-cell cloud) is counted in
-// a host-cell grid when all masses are equal and spread by the 27-point
-// stencil at the end; every other hit deposits its clipped cloud with the
-// 32 lanes of the warp, hits with the same host cell, level and mass once
-// with the group size as factor.
+// Work unit: PZ z-planes of one patch.  A unit's candidates are the particles
+// of the bins that overlap the patch box extended by MAXKERNELEXT = DX
+// (grids.f:837-893), restricted in z to the unit's planes +- DX; they are split
+// into slices of PSLICE so that a dense unit is shared by several CTAs, whose
+// sums meet in a float64 scratch slab.
 #define PZ 4              // z planes per unit
 #define PZ_BLOCK 256
 #define NSLAB (NA / PZ)
-#define PSLICE 8192       // candidates per work item
+#define PSLICE 24576      // candidates per work item: counts of a slice fit 16 bits (of 8192, 16384, 24576 and
+                          // 32768, the equal-mass kernel measured 17.5, 16.3, 15.9, 15.7 ms at 384^3)
 #define PROWS 128         // bin rows staged in shared memory at a time
-#define CGX (NA + 2)      // host-cell count grid: x, y in [0, NA+1]
 #define AROW (NA + 5)     // accumulator row stride (doubles): rows shifted by 5 banks pairs
 #define APLANE (NA * AROW)
 #define ACC_N (PZ * APLANE)
-#define CGZ (PZ + 2)      //                       z in [zlo-1, zhi+1]
 
 // Offset of the centre of level l in the compact kernel table that stores
 // levels 0, 1, ... back to back (2*2^l+1 entries each).
@@ -955,19 +953,359 @@ static int unit_list_fill(asohf_ctx* c, const UnitList& U, int unit_cells, FW wa
   return ASOHF_OK;
 }
 
-// One work item (a slice of one 4-plane unit of a patch) of the patch deposit.
-__device__ __forceinline__ void density_patch_item(const int2 it, const DevMesh& M, const Bins& B,
-                                                   const float4* __restrict__ P, const uint8_t* __restrict__ S,
-                                                   const int32_t* __restrict__ order, const PatchWork& W, float dx,
-                                                   const float* __restrict__ kernels, int eqmass,
-                                                   float* __restrict__ u11, const float* __restrict__ denbas_lev) {
-  extern __shared__ double acc[];  // ACC_N doubles (padded rows), count grid, kernel table
-  int32_t* scnt = (int32_t*)(acc + ACC_N);
-  float* ktab = (float*)(scnt + CGX * CGX * CGZ);
+// One work item (a slice of one PZ-plane unit of a patch), equal masses.  The
+// unit's sums live in registers: lane i of warp w holds cells (i, 4w .. 4w+3,
+// every plane) in float64, so clouds are added without atomics.  Hosts of level
+// 0 and 1 (most hits) are counted, both levels in the halves of one word a cell
+// (a slice holds at most PSLICE hosts, so no half and no sum of counts
+// overflows), and spread by a stencil at the end: with a kernel symmetric in
+// each axis the (2r+1)^3 terms of a level take (r+1)^3 values t(|di|, |dj|,
+// |dk|), each formed once.  Wider clouds are listed by the scan and added by
+// the warps whose rows they meet.
+//
+// Float64 conversions run at 16 lanes a clock and SM and shared-memory float64
+// atomics (compare and swap) at 4.7, additions at 61.  A positive normal REAL*4
+// term is widened by one integer product, its bits times 2^29, which is the
+// term times 2^-896 exactly; the sums are scaled back at the end.
+//
+// Measured at 56.6M particles, 12012 patches (96096 units, 698M candidates, 166M
+// hits): 15.9 ms; 21.7 ms with every hit above level 0 added by shared-memory
+// atomics.  About 6 ms are the scan, 4.5 the level-2 clouds, 2.6 the stencil, 2
+// the wider clouds, 1.5 clearing and writing; bound by instruction issue and
+// the latency of short lists (24 warps an SM, registers and shared memory).
+#define SCALE_UP 0x1p896
+#define CG (NA + 4)               // count grid rows: x, y in [-1, NA+2]
+#define CGP (PZ + 4)              // its planes, z in [zlo-2, zhi+2]
+#define ROUND (PZ_BLOCK * 2)      // candidates scanned between two looks at the lists
+#define LCAP (2 * ROUND)          // listed clouds, added when another round might not fit
+// Level-2 clouds of one mass (9^3 cells, the most of the listed ones): their
+// terms as a table t[|di|][|dj|][dk], 0 past the cloud, 4 copies shifted by a
+// plane each so that the terms of a unit's 4 planes are one 16-byte read, and
+// their list sorted by (eighth columns, quarter rows) of the host.  A cloud of
+// columns 8b-7 .. 8b+8 leaves most of a warp's 32 columns idle, so a warp adds
+// clouds of the host blocks 0, 2, 4 together, each on its own lanes, then those
+// of blocks 1 and 3.
+#define T2R 20                    // floats a row of the table: 16 used, banks spread
+#define T2A (6 * T2R)
+#define T2COPY (6 * T2A)
+#define NB2 50                    // 5 column blocks of 8 hosts x 10 row blocks of 4
+
+__device__ __forceinline__ double widen(float t) {
+  unsigned long long w;
+  asm("mul.wide.u32 %0, %1, 0x20000000;" : "=l"(w) : "r"(__float_as_uint(t)));
+  return __longlong_as_double((long long)w);
+}
+
+// a count below 2^32 as float64: the low word of 2^52 + v
+__device__ __forceinline__ double count_d(uint32_t v) {
+  return __hiloint2double(0x43300000, (int)v) - 4503599627370496.0;
+}
+
+// floor(v / d) of the rounded quotient: the product with rd = 1/d, below 1000
+// within 3e-4 of it, decides unless it lies within 1e-3 of an integer
+__device__ __forceinline__ int floor_div(float v, float d, float rd) {
+  const float r = v * rd;
+  float f = floorf(r);
+  if (fabsf(r - rintf(r)) < 1e-3f || fabsf(r) > 1000.0f) f = floorf(v / d);
+  return (int)f;
+}
+
+__global__ void __launch_bounds__(PZ_BLOCK, 3)
+k_density_patches_eq(DevMesh M, Bins B, const float4* __restrict__ P, const int32_t* __restrict__ order, PatchWork W,
+                     float dx, const float* __restrict__ kernels,
+                     float meq, const float* __restrict__ t2g, float* __restrict__ u11,
+                     const float* __restrict__ denbas_lev) {
+  extern __shared__ uint4 dyn[];
+  uint32_t* cnt = (uint32_t*)dyn;             // counts[CGP][CG][CG]
+  float* t2 = (float*)(cnt + CGP * CG * CG);  // the level-2 table
+  float* ktab = t2 + 4 * T2COPY;              // the kernels
+  __shared__ int s_lo[PROWS], s_pre[PROWS + 1], s_nlist, s_any[2];
+  __shared__ unsigned long long s_list[LCAP];
+  __shared__ double s_t0[8], s_t1[27];
+  __shared__ unsigned short s_l2[LCAP], s_l2s[LCAP + 1];  // listed level-2 clouds, and sorted
+  __shared__ int s_nl2, s_off2[NB2 + 1], s_cur2[NB2];
+  const unsigned FULL = 0xffffffffu;
+  const int2 it = W.items[blockIdx.x];
+  UnitGeo g;
+  unit_geo(M, B, order, it.x, dx, g);
+  float* out = u11 + (size_t)g.ip * NA * NA * NA + (size_t)g.slab * PZ * NA * NA;
+  if (g.zlo > g.zhi) {  // planes past the patch
+    for (int q = threadIdx.x; q < NA * NA * PZ; q += blockDim.x) out[q] = 0.0f;
+    return;
+  }
+  for (int q = threadIdx.x; q < CGP * CG * CG; q += blockDim.x) cnt[q] = 0;
+  for (int l = 0; l <= g.ir; l++) {
+    int nk = 1 << l, c0 = ktab_center(l);
+    for (int i = threadIdx.x - nk; i <= nk; i += blockDim.x)
+      ktab[c0 + i] = kernels[(size_t)l * KW + ASOHF_NMAX_KERNELS + i];
+  }
+  if (threadIdx.x < 2) s_any[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_nlist = s_nl2 = 0;
+  __syncthreads();
+  if (threadIdx.x < 35) {  // the distinct terms of levels 0 and 1
+    const int l = threadIdx.x < 27 ? 1 : 0, q = l ? threadIdx.x : threadIdx.x - 27, b = l ? 3 : 2;
+    if (l <= g.ir) {
+      const float* kc = ktab + ktab_center(l);
+      (l ? s_t1 : s_t0)[q] =
+          widen(__fmul_rn(__fmul_rn(__fmul_rn(meq, kc[q % b]), kc[(q / b) % b]), kc[q / (b * b)]));
+    }
+  }
+  if (g.ir >= 2)
+    for (int q = threadIdx.x; q < T2COPY; q += blockDim.x) ((float4*)t2)[q] = ((const float4*)t2g)[q];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int j0 = 4 * warp + 1;  // the warp's rows j0 .. j0+3
+  double acc[4][PZ];
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int p = 0; p < PZ; p++) acc[q][p] = 0.0;
+  const float rdx = 1.0f / g.dxpa;
+  // the listed clouds on the warp's rows
+  auto add_listed = [&](int nl) {
+    for (int e0 = 0; e0 < nl; e0 += 32) {
+      unsigned todo = 0;
+      {
+        bool mine = false;
+        if (e0 + lane < nl) {
+          const unsigned long long e = s_list[e0 + lane];
+          const int jy = (int)((e >> 32) & 0xffff) - 1024, nk = 1 << (int)(e & 0xffff);
+          mine = jy - nk <= j0 + 3 && jy + nk >= j0 && j0 <= g.n2;
+        }
+        todo = __ballot_sync(FULL, mine);
+      }
+      while (todo) {
+        const int src = e0 + __ffs(todo) - 1;
+        todo &= todo - 1;
+        const unsigned long long e = s_list[src];
+        const int ix = (int)(e >> 48) - 1024, jy = (int)((e >> 32) & 0xffff) - 1024;
+        const int kz = (int)((e >> 16) & 0xffff) - 1024, lev = (int)(e & 0xffff), nk = 1 << lev;
+        const float* kc = ktab + ktab_center(lev);
+        const int ox = lane + 1 - ix;
+        const float bx = ox >= -nk && ox <= nk ? __fmul_rn(meq, kc[ox]) : 0.0f;
+        float wz[PZ];
+#pragma unroll
+        for (int p = 0; p < PZ; p++) {
+          const int oz = g.zlo + p - kz;
+          wz[p] = oz >= -nk && oz <= nk ? kc[oz] : 0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const int oy = j0 + q - jy;
+          if (oy >= -nk && oy <= nk) {
+            const float bw = __fmul_rn(bx, kc[oy]);
+#pragma unroll
+            for (int p = 0; p < PZ; p++) acc[q][p] += widen(__fmul_rn(bw, wz[p]));
+          }
+        }
+      }
+    }
+  };
+  // the level-2 list: counting sort by block, then every warp its three row
+  // blocks (hosts within 4 rows of its own), several column blocks at a time
+  auto add_level2 = [&](int n) {
+    if (n == 0) return;
+    for (int q = threadIdx.x; q < NB2; q += blockDim.x) s_cur2[q] = 0;
+    __syncthreads();
+    auto block = [](unsigned e) { return (int)((e >> 13) * 10 + ((e >> 6) & 15)); };
+    for (int q = threadIdx.x; q < n; q += blockDim.x) atomicAdd(&s_cur2[block(s_l2[q])], 1);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      int run = 0;
+      for (int q = lane; q - lane < NB2; q += 32) {
+        const int v = q < NB2 ? s_cur2[q] : 0;
+        int sc = v;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(FULL, sc, o);
+          if (lane >= o) sc += y;
+        }
+        if (q < NB2) s_off2[q] = s_cur2[q] = run + sc - v;
+        run += __shfl_sync(FULL, sc, 31);
+      }
+      if (lane == 0) s_off2[NB2] = run;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < n; q += blockDim.x) {
+      const unsigned short e = s_l2[q];
+      s_l2s[atomicAdd(&s_cur2[block(e)], 1)] = e;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int phase = 0; phase < 2; phase++) {
+      const int bin = phase == 0 ? (lane < 8 ? 0 : (lane < 24 ? 2 : 4)) : (lane < 16 ? 1 : 3);
+      const int lo = s_off2[bin * 10 + warp], len = s_off2[bin * 10 + warp + 3] - lo;
+      const int most = __reduce_max_sync(FULL, len);
+      for (int q = 0; q < most; q++) {
+        const unsigned e = s_l2s[q < len ? lo + q : lo];
+        const int a = q < len ? min(abs(lane + 4 - (int)(e >> 10)), 5) : 5;
+        const int dz = 11 - (int)(e & 15), dj = j0 + 3 - (int)((e >> 4) & 63);
+        const float* t = t2 + (dz & 3) * T2COPY + a * T2A + (dz & ~3);
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const float4 v = *(const float4*)(t + min(abs(dj + r), 5) * T2R);
+          acc[r][0] += widen(v.x);
+          acc[r][1] += widen(v.y);
+          acc[r][2] += widen(v.z);
+          acc[r][3] += widen(v.w);
+        }
+      }
+    }
+  };
+  const int64_t v0 = (int64_t)it.y * PSLICE, v1 = v0 + PSLICE;
+  int64_t vbase = 0;
+  for (int r0 = 0; r0 < g.rows; r0 += PROWS) {
+    const int nr = min(PROWS, g.rows - r0);
+    __syncthreads();
+    stage_rows(B, g, r0, nr, s_lo, s_pre);
+    __syncthreads();
+    const int tot = s_pre[nr];
+    const int b = (int)(min(v1, vbase + tot) - vbase);
+    const int a = (int)(max(v0, vbase) - vbase);
+    for (int rb = a; rb < b; rb += ROUND) {  // 64 candidates a warp
+      const int cb = rb + warp * 64, ce = min(cb + 63, b - 1);
+      if (cb <= ce) {
+        // rows of the warp's first and last candidates
+        int c0 = 0, c1 = 0;
+        for (int r = 1 + lane; r <= nr; r += 32) {
+          const int sp = s_pre[r];
+          c0 += sp <= cb;
+          c1 += sp <= ce;
+        }
+        int row0 = (int)__reduce_add_sync(FULL, (unsigned)c0);
+        const int row1 = (int)__reduce_add_sync(FULL, (unsigned)c1);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int v = cb + 32 * h + lane;
+          int ix = 0, jy = 0, kz = 0, lev = -1;
+          if (v <= ce) {
+            int row = row0, hi = row1;
+            while (row < hi) {
+              const int mid = (row + hi + 1) >> 1;
+              if (s_pre[mid] <= v) row = mid; else hi = mid - 1;
+            }
+            row0 = row;
+            const int e = s_lo[row] + (v - s_pre[row]);
+            const float4 q = P[e];
+            const int s = __float_as_int(q.w);
+            if (s != 255 && g.pxl < q.x && q.x < g.pxr && g.pyl < q.y && q.y < g.pyr && g.pzl < q.z && q.z < g.pzr) {
+              const int l = max(g.ir - s, 0), nk = 1 << l;
+              ix = floor_div(q.x - g.xlfix, g.dxpa, rdx) + 1;
+              jy = floor_div(q.y - g.ylfix, g.dxpa, rdx) + 1;
+              kz = floor_div(q.z - g.zlfix, g.dxpa, rdx) + 1;
+              if (!(ix - nk > g.n1 || ix + nk < 1 || jy - nk > g.n2 || jy + nk < 1) && kz - nk <= g.zhi &&
+                  kz + nk >= g.zlo) {
+                lev = l;
+              }
+            }
+          }
+          if (lev == 0 || lev == 1) {
+            atomicAdd(&cnt[((kz - g.zlo + 2) * CG + (jy + 1)) * CG + (ix + 1)], lev ? 0x10000u : 1u);
+            s_any[lev] = 1;
+          }
+          {
+            const unsigned two = __ballot_sync(FULL, lev == 2);
+            if (two) {
+              int o = 0;
+              if (lane == 0) o = atomicAdd(&s_nl2, __popc(two));
+              o = __shfl_sync(FULL, o, 0) + __popc(two & ((1u << lane) - 1u));
+              if (lev == 2)
+                s_l2[o] = (unsigned short)(((ix + 3) << 10) | ((jy + 3) << 4) | (kz - g.zlo + 4));
+            }
+            if (lev == 2) lev = -1;
+          }
+          const unsigned wide = __ballot_sync(FULL, lev >= 2);
+          if (wide) {
+            int o = 0;
+            if (lane == 0) o = atomicAdd(&s_nlist, __popc(wide));
+            o = __shfl_sync(FULL, o, 0) + __popc(wide & ((1u << lane) - 1u));
+            if (lev >= 2) {
+              s_list[o] = (unsigned long long)(uint32_t)(((ix + 1024) << 16) | (jy + 1024)) << 32 |
+                          (uint32_t)(((kz + 1024) << 16) | lev);
+            }
+          }
+        }
+      }
+      __syncthreads();
+      const int nl = s_nlist, nl2 = s_nl2;
+      __syncthreads();
+      if (nl > LCAP - ROUND || nl2 > LCAP - ROUND) {
+        add_listed(nl);
+        add_level2(nl2);
+        __syncthreads();
+        if (threadIdx.x == 0) s_nlist = s_nl2 = 0;
+        __syncthreads();
+      }
+    }
+    vbase += tot;
+  }
+  __syncthreads();
+  add_listed(s_nlist);
+  add_level2(s_nl2);
+  if (s_any[0] | s_any[1]) {
+    const bool any0 = s_any[0] != 0, any1 = s_any[1] != 0;
+#pragma unroll 1
+    for (int a = 0; a < 3; a++) {  // |di|
+#pragma unroll
+      for (int pl = 0; pl < CGP; pl++) {
+        uint32_t X[8];  // rows j0-2 .. j0+5: the counts at -a and +a
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+          const uint32_t* c = cnt + (pl * CG + (4 * warp + r)) * CG + lane + 2;
+          X[r] = a == 0 ? c[0] : c[-a] + c[a];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+          for (int bb = 0; bb < 3; bb++) {  // |dj|
+            const uint32_t Y = bb == 0 ? X[q + 2] : X[q + 2 - bb] + X[q + 2 + bb];
+            if (any1) {
+              const double d1 = count_d(Y >> 16);
+#pragma unroll
+              for (int p = 0; p < PZ; p++) {
+                const int gz = pl - 2 - p < 0 ? p + 2 - pl : pl - 2 - p;  // |dk|
+                if (gz <= 2) acc[q][p] = __fma_rn(d1, s_t1[gz * 9 + bb * 3 + a], acc[q][p]);
+              }
+            }
+            if (any0 && bb < 2 && a < 2 && pl >= 1 && pl <= CGP - 2) {
+              const double d0 = count_d(Y & 0xffffu);
+#pragma unroll
+              for (int p = 0; p < PZ; p++) {
+                const int gz = pl - 2 - p < 0 ? p + 2 - pl : pl - 2 - p;
+                if (gz <= 1) acc[q][p] = __fma_rn(d0, s_t0[gz * 4 + bb * 2 + a], acc[q][p]);
+              }
+            }
+          }
+      }
+    }
+  }
+  const int sidx = W.scratch_of[it.x];
+  const float den = denbas_lev[g.ir];
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int p = 0; p < PZ; p++) {
+      const int j = j0 - 1 + q, at = (p * NA + j) * NA + lane;  // 0-based cell (lane, j, slab*PZ + p)
+      const double s = acc[q][p] * SCALE_UP;
+      if (sidx < 0)
+        out[at] = lane < g.n1 && j < g.n2 && g.slab * PZ + p < g.n3 ? (float)s / den : 0.0f;
+      else if (s != 0.0)  // one slice of a shared unit
+        atomicAdd(&W.scratch[(size_t)sidx * NA * NA * PZ + at], s);
+    }
+}
+
+// One work item, any masses: float64 sums in shared memory, one cloud a warp
+// step, hits with the same host cell, level and mass once with their number as
+// factor.  (The registers and lists of the equal-mass kernel measured slower
+// here, 1.64 against 1.24 ms for 1.4M particles of two masses on 888 patches:
+// without counts and tables every hit is listed or added by itself.)
+__global__ void __launch_bounds__(PZ_BLOCK, 3)
+k_density_patches(DevMesh M, Bins B, const float4* __restrict__ P, const uint8_t* __restrict__ S,
+                  const int32_t* __restrict__ order, PatchWork W, float dx, const float* __restrict__ kernels,
+                  float* __restrict__ u11, const float* __restrict__ denbas_lev) {
+  extern __shared__ double acc[];  // ACC_N doubles (padded rows), kernel table
+  float* ktab = (float*)(acc + ACC_N);
+  const int2 it = W.items[blockIdx.x];
   __shared__ int s_lo[PROWS], s_pre[PROWS + 1], s_next;
-  __shared__ double s_t27[27];
   __shared__ float s_rcp[NA + 1];  // 1/n for the clipped cloud widths n <= NA
-  __shared__ int s_any;            // some level-0 host was counted
   UnitGeo g;
   unit_geo(M, B, order, it.x, dx, g);
   float* out = u11 + (size_t)g.ip * NA * NA * NA + (size_t)g.slab * PZ * NA * NA;
@@ -976,50 +1314,21 @@ __device__ __forceinline__ void density_patch_item(const int2 it, const DevMesh&
     return;
   }
   for (int q = threadIdx.x; q < ACC_N; q += blockDim.x) acc[q] = 0.0;
-  for (int q = threadIdx.x; q < CGX * CGX * CGZ; q += blockDim.x) scnt[q] = 0;
   for (int l = 0; l <= g.ir; l++) {
     int nk = 1 << l, c0 = ktab_center(l);
     for (int i = threadIdx.x - nk; i <= nk; i += blockDim.x)
       ktab[c0 + i] = kernels[(size_t)l * KW + ASOHF_NMAX_KERNELS + i];
   }
   if (threadIdx.x >= 1 && threadIdx.x <= NA) s_rcp[threadIdx.x] = 1.0f / (float)threadIdx.x;
-  if (threadIdx.x == 0) s_any = 0;
   __syncthreads();
-  if (eqmass && threadIdx.x < 27) {  // level-0 terms of the common mass
-    const float* kc = ktab + ktab_center(0);
-    float m0 = P[0].w;  // any staged particle: all masses are equal
-    int a = threadIdx.x % 3 - 1, b = (threadIdx.x / 3) % 3 - 1, cc = threadIdx.x / 9 - 1;
-    s_t27[threadIdx.x] = (double)__fmul_rn(__fmul_rn(__fmul_rn(m0, kc[a]), kc[b]), kc[cc]);
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   const int64_t v0 = (int64_t)it.y * PSLICE, v1 = v0 + PSLICE;
   int64_t vbase = 0;
   for (int r0 = 0; r0 < g.rows; r0 += PROWS) {
     int nr = min(PROWS, g.rows - r0);
     __syncthreads();
-    if (threadIdx.x < nr) {
-      int lo, len;
-      row_range(B, g, r0 + threadIdx.x, &lo, &len);
-      s_lo[threadIdx.x] = lo;
-      s_pre[threadIdx.x + 1] = len;
-    }
-    __syncthreads();
-    if (warp == 0) {  // inclusive prefix of the row lengths in place, 32 rows at a time
-      int run = 0;
-      for (int r = 1 + lane; r - lane <= nr; r += 32) {
-        int sc = r <= nr ? s_pre[r] : 0;
-        for (int o = 1; o < 32; o <<= 1) {
-          int y = __shfl_up_sync(0xffffffffu, sc, o);
-          if (lane >= o) sc += y;
-        }
-        if (r <= nr) s_pre[r] = run + sc;
-        run += __shfl_sync(0xffffffffu, sc, 31);
-      }
-      if (lane == 0) {
-        s_pre[0] = 0;
-        s_next = (int)(max(v0, vbase) - vbase);  // first candidate of this slice in these rows
-      }
-    }
+    stage_rows(B, g, r0, nr, s_lo, s_pre);
+    if (threadIdx.x == 0) s_next = (int)(max(v0, vbase) - vbase);  // this slice's first candidate in these rows
     __syncthreads();
     const int tot = s_pre[nr];
     const int b = (int)(min(v1, vbase + tot) - vbase);
@@ -1062,12 +1371,7 @@ __device__ __forceinline__ void density_patch_item(const int2 it, const DevMesh&
           if (!(ix - nk > g.n1 || ix + nk < 1 || jy - nk > g.n2 || jy + nk < 1 || kz - nk > g.n3 || kz + nk < 1) &&
               max(max(kz - nk, 1), g.zlo) <= min(min(kz + nk, g.n3), g.zhi)) {
             mp = q.w;
-            if (eqmass && lev == 0) {  // host cell count (ix in [0, n1+1], kz in [zlo-1, zhi+1])
-              atomicAdd(&scnt[((kz - g.zlo + 1) * CGX + jy) * CGX + ix], 1);
-              s_any = 1;
-            } else {
-              hit = true;
-            }
+            hit = true;
           }
         }
       }
@@ -1133,54 +1437,6 @@ __device__ __forceinline__ void density_patch_item(const int2 it, const DevMesh&
     vbase += tot;
   }
   __syncthreads();
-  // level-0 hosts: 27-point stencil of the counts (cells inside the patch)
-  if (eqmass && s_any && ktab[ktab_center(0) - 1] == ktab[ktab_center(0) + 1]) {
-    // a symmetric level-0 kernel leaves 8 distinct terms, t(|di|, |dj|, |dk|):
-    // a thread takes a column of cells, sums the counts of each neighbour
-    // pattern plane by plane (integers) and forms 8 products per cell
-    double tp[8];
-#pragma unroll
-    for (int q = 0; q < 8; q++) tp[q] = s_t27[((q >> 2) + 1) * 9 + (((q >> 1) & 1) + 1) * 3 + ((q & 1) + 1)];
-    for (int col = threadIdx.x; col < NA * NA; col += blockDim.x) {
-      const int i = col % NA + 1, j = col / NA + 1;
-      if (i > g.n1 || j > g.n2) continue;
-      int a0[CGZ], ax[CGZ], ay[CGZ], axy[CGZ];  // per count plane: centre, x pair, y pair, corners
-#pragma unroll
-      for (int pz = 0; pz < CGZ; pz++) {
-        const int32_t* r0 = scnt + (pz * CGX + j) * CGX + i;
-        const int32_t* rm = r0 - CGX;
-        const int32_t* rp = r0 + CGX;
-        a0[pz] = r0[0];
-        ax[pz] = r0[-1] + r0[1];
-        ay[pz] = rm[0] + rp[0];
-        axy[pz] = (rm[-1] + rm[1]) + (rp[-1] + rp[1]);
-      }
-#pragma unroll
-      for (int pz = 1; pz <= PZ; pz++) {  // output plane k = zlo + pz - 1
-        if (g.zlo + pz - 1 > g.zhi) break;
-        const int c0 = a0[pz], c1 = ax[pz], c2 = ay[pz], c3 = axy[pz];
-        const int c4 = a0[pz - 1] + a0[pz + 1], c5 = ax[pz - 1] + ax[pz + 1];
-        const int c6 = ay[pz - 1] + ay[pz + 1], c7 = axy[pz - 1] + axy[pz + 1];
-        if ((c0 | c1 | c2 | c3 | c4 | c5 | c6 | c7) == 0) continue;
-        double s = (double)c0 * tp[0] + (double)c1 * tp[1] + (double)c2 * tp[2] + (double)c3 * tp[3] +
-                   (double)c4 * tp[4] + (double)c5 * tp[5] + (double)c6 * tp[6] + (double)c7 * tp[7];
-        acc[(pz - 1) * APLANE + (j - 1) * AROW + (i - 1)] += s;
-      }
-    }
-  } else if (eqmass && s_any) {
-    for (int q = threadIdx.x; q < NA * NA * PZ; q += blockDim.x) {
-      int i = q % NA + 1, j = (q / NA) % NA + 1, k = g.zlo + q / (NA * NA);
-      if (i > g.n1 || j > g.n2 || k > g.zhi) continue;
-      double s = 0.0;
-      for (int kk = -1; kk <= 1; kk++)
-        for (int jj = -1; jj <= 1; jj++)
-          for (int ii = -1; ii <= 1; ii++) {
-            int c = scnt[((k - kk - g.zlo + 1) * CGX + (j - jj)) * CGX + (i - ii)];
-            if (c) s += (double)c * s_t27[(kk + 1) * 9 + (jj + 1) * 3 + (ii + 1)];
-          }
-      acc[(k - g.zlo) * APLANE + (j - 1) * AROW + (i - 1)] += s;
-    }
-  }
   const int sidx = W.scratch_of[it.x];
   if (sidx < 0) {
     __syncthreads();
@@ -1198,26 +1454,6 @@ __device__ __forceinline__ void density_patch_item(const int2 it, const DevMesh&
       double a = acc[(q / (NA * NA)) * APLANE + ((q / NA) % NA) * AROW + q % NA];
       if (a != 0.0) atomicAdd(&sc[q], a);
     }
-  }
-}
-
-// The patch deposit over its work items: CTA b takes item b, and, with a
-// work counter (a grid smaller than the item count), the next free item
-// after each one.
-__global__ void __launch_bounds__(PZ_BLOCK, 3)
-k_density_patches(DevMesh M, Bins B, const float4* __restrict__ P, const uint8_t* __restrict__ S,
-                  const int32_t* __restrict__ order, PatchWork W, float dx, const float* __restrict__ kernels,
-                  int eqmass, float* __restrict__ u11, const float* __restrict__ denbas_lev, int nitems,
-                  int* __restrict__ next_item) {
-  __shared__ int s_item;
-  int item = blockIdx.x;
-  while (item < nitems) {
-    density_patch_item(W.items[item], M, B, P, S, order, W, dx, kernels, eqmass, u11, denbas_lev);
-    if (!next_item) break;
-    __syncthreads();  // the item's last reads of shared memory are done
-    if (threadIdx.x == 0) s_item = atomicAdd(next_item, 1) + (int)gridDim.x;
-    __syncthreads();
-    item = s_item;
   }
 }
 
@@ -1294,14 +1530,14 @@ extern "C" int asohf_density(asohf_ctx* c, int nx, float lado0, float dx, float 
   const bool defer = c->density_overlap && on_device && np > 0 && n > 0 && c->dens_stream;
   const DAlloc A{c, defer};
   size_t need = 12 * g + (on_device ? 0 : 4 * g + 4 * (size_t)np * NA * NA * NA) +
-                4 * KW * (ASOHF_NLEVELS + 1) + 96 * (size_t)np + 16384 +
+                4 * KW * (ASOHF_NLEVELS + 1) + 16 * T2COPY + 96 * (size_t)np + 16384 +
                 (np ? bins_bytes(nall, lado0, dx, 2) + 17 * (size_t)nall + unit_list_bytes(NSLAB * np) +
                           4 * NSLAB * (size_t)np : 0);
   ASOHF_CHECK(arena_reserve(c, need));
   if (defer) {  // what the deferred kernels read: kernels, mesh, order, bins, staged particles, renorm dims
     const int nbw = (int)lrintf(lado0 / dx);
     const int64_t nb = (nbw + 1) / 2, nbin = nb * nb * nb;
-    ASOHF_CHECK(dpool_reserve(c, 0, 4 * KW * (ASOHF_NLEVELS + 1) + 4 * (ASOHF_NLEVELS + 1) + 48 * (size_t)np +
+    ASOHF_CHECK(dpool_reserve(c, 0, 4 * KW * (ASOHF_NLEVELS + 1) + 16 * T2COPY + 4 * (ASOHF_NLEVELS + 1) + 48 * (size_t)np +
                                         4 * (size_t)(nbin + 1) + 17 * (size_t)nall + 4 * NSLAB * (size_t)np +
                                         16 * 256));
   }
@@ -1319,6 +1555,34 @@ extern "C" int asohf_density(asohf_ctx* c, int nx, float lado0, float dx, float 
         t = t * h0[kk];
         T27.t[(kk + 1) * 9 + (jj + 1) * 3 + (ii + 1)] = (double)t;
       }
+  // the counting patch kernel: one mass, and every term of every level normal
+  bool pd_eq = eqmass;
+  for (int ir = 0; ir <= nl; ir++) {
+    const float e = hk[(size_t)ir * KW + ASOHF_NMAX_KERNELS + (1 << ir)];
+    volatile float t = c->norma * e;
+    t = t * e;
+    t = t * e;
+    if (!(t >= 1.17549435e-38f)) pd_eq = false;
+  }
+  float* dt2 = nullptr;  // level-2 terms, t[copy][|di|][|dj|][dk], 0 past the cloud
+  std::vector<float> ht2;
+  if (pd_eq && nl >= 2) {
+    const float* k2 = hk + 2 * KW + ASOHF_NMAX_KERNELS;
+    ht2.assign(4 * T2COPY, 0.0f);
+    for (int cp = 0; cp < 4; cp++)
+      for (int a = 0; a <= 4; a++)
+        for (int b = 0; b <= 4; b++)
+          for (int oz = -4; oz <= 4; oz++) {
+            const int e = oz + 7 - cp;
+            if (e > 15) continue;
+            volatile float t = c->norma * k2[a];
+            t = t * k2[b];
+            t = t * k2[oz];
+            ht2[cp * T2COPY + a * T2A + b * T2R + e] = t;
+          }
+    dt2 = upload_floats(c, ht2.data(), ht2.size(), A);
+    if (!dt2) return ASOHF_ERR_CAPACITY;
+  }
   bool sym27 = true;  // each term equals the one of its mirrored offsets
   for (int q = 0; q < 27; q++) {
     const int ii = q % 3 - 1, jj = (q / 3) % 3 - 1, kk = q / 9 - 1;
@@ -1397,7 +1661,7 @@ extern "C" int asohf_density(asohf_ctx* c, int nx, float lado0, float dx, float 
         int kt_ = ktime_begin(c, "density_bin_stage");
         k_bin_stage<<<grid_for(nall, 256, c->num_sms * 16), 256, 0, c->stream>>>(
             B.idx, nall, n, c->p.x, c->p.y, c->p.z, c->p.m, c->rows_cur >= 0 ? c->rows[c->rows_cur] : nullptr,
-            dend, bp, bs);
+            dend, bp, bs, pd_eq ? 1 : 0);
         k_patch_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, order, nunits, dx, U.key, U.unit);
         ktime_end(c, kt_);
         c->launches += 2;
@@ -1412,13 +1676,10 @@ extern "C" int asohf_density(asohf_ctx* c, int nx, float lado0, float dx, float 
       ASOHF_CHECK(unit_list_fill(c, U, NA * NA * PZ,
                                  [&](size_t b) { return defer ? dpool_alloc(c, 1, b) : seg_alloc(c, b); },
                                  [&](size_t b) { return A.get(b); }, &W, &dmulti));
-      // one CTA per item; the kernel can also run as a smaller grid drawing
-      // items from a counter (next_item), which measured slower beside the
-      // halo finder (the patch deposit took 181 ms as one CTA per SM and
-      // slowed the halo kernels by 38 ms), so the full grid is launched
-      int* next_item = nullptr;
-      size_t smem = sizeof(double) * ACC_N + sizeof(int32_t) * CGX * CGX * CGZ + sizeof(float) * ktab_size(nl);
-      ASOHF_CUDA(cudaFuncSetAttribute(k_density_patches, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      const size_t smem = (pd_eq ? sizeof(uint32_t) * CGP * CG * CG + sizeof(float) * 4 * T2COPY
+                                 : sizeof(double) * ACC_N) + sizeof(float) * ktab_size(nl);
+      ASOHF_CUDA(cudaFuncSetAttribute(pd_eq ? (const void*)k_density_patches_eq : (const void*)k_density_patches,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       // deferred: the patch kernels run on the density stream after the
       // staging above, and the call returns without waiting for them
       cudaStream_t ps = c->stream;
@@ -1428,8 +1689,11 @@ extern "C" int asohf_density(asohf_ctx* c, int nx, float lado0, float dx, float 
         ps = c->dens_stream;
       }
       int kt_ = ktime_begin(c, "density_patches", ps);
-      k_density_patches<<<(unsigned)U.nitems, PZ_BLOCK, smem, ps>>>(M, B, bp, bs, order, W, dx, dk, eqmass ? 1 : 0,
-                                                               du11, dden, U.nitems, next_item);
+      if (pd_eq)
+        k_density_patches_eq<<<(unsigned)U.nitems, PZ_BLOCK, smem, ps>>>(M, B, bp, order, W, dx, dk, c->norma, dt2,
+                                                                         du11, dden);
+      else
+        k_density_patches<<<(unsigned)U.nitems, PZ_BLOCK, smem, ps>>>(M, B, bp, bs, order, W, dx, dk, du11, dden);
       if (U.nmulti) k_patch_finish<<<U.nmulti, 256, 0, ps>>>(M, order, dmulti, W.scratch, du11, dden);
       ktime_end(c, kt_, ps);
       c->launches += 1 + (U.nmulti > 0);
@@ -1838,7 +2102,7 @@ extern "C" int asohf_interpolate_density_tsc(asohf_ctx* c, int nx, float lado0, 
     int kt_ = ktime_begin(c, "tsc_base");
     k_bin_stage<<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(
         B.idx, n, n, c->p.x, c->p.y, c->p.z, c->p.m, c->rows_cur >= 0 ? c->rows[c->rows_cur] : nullptr, nullptr, bp,
-        nullptr);
+        nullptr, 0);
     k_tsc_base_runs<<<grid_for(n, TSC_BLOCK, c->num_sms * 8), TSC_BLOCK, 0, c->stream>>>(bp, n, nx, xl, dx, dradx,
                                                                                          acc);
     ktime_end(c, kt_);
