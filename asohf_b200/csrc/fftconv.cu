@@ -8,17 +8,18 @@
 // R2C, a separate multiply and a 3-D C2R, the z transforms and the multiply
 // share one read and one write of the spectrum.
 //
-// Line transforms are done by one warp: an M = 32 R point line is held as
-// R values per lane (lane l, register n1 = element l + 32 n1), transformed
-// by an R-point decimation-in-frequency FFT in registers, a twiddle W_M^(l k1)
-// and a 32-point decimation-in-frequency FFT across lanes (shuffles); lane l
-// register p then holds frequency brev_R(p) + R brev_5(l).  The Green's
-// factor is applied in that order and the inverse transform (the same
-// stages undone in reverse, decimation in time) returns natural order, so
-// the line goes through shared memory only on its way in and out.
-// Twiddles W_N^j are a table computed on the host in double precision.  The
-// result equals an FFT-based solve within float32 rounding (not bit for bit
-// a library's).
+// A line of N = V T values is transformed by T threads in two register
+// passes with one exchange through shared memory.  Thread s holds elements
+// s + T n1 (n1 < V): a V-point FFT over n1 gives A[k1], the exchange hands
+// thread k1 mod T the values A_s[k1] of every s, which it turns by W_N^(s k1)
+// and transforms over s into the frequencies k1 + V k2.  The Green's factor is
+// applied there, and the same steps undone in reverse order return natural
+// order; each thread writes its groups back where it read them, so the
+// exchange buffer needs two barriers in all.  Register FFTs are decimation in
+// frequency forward (output in bit-reversed order) and decimation in time
+// back (input in bit-reversed order), so nothing is permuted.  Twiddles W_N^j
+// are a table computed on the host in double precision.  The result equals an
+// FFT-based solve within float32 rounding (not bit for bit a library's).
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -28,8 +29,6 @@
 
 namespace {
 
-constexpr unsigned FULL = 0xffffffffu;
-
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 // complex product with fused multiply-adds (two roundings per part)
@@ -37,11 +36,6 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
   return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
 __device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }
-
-// index of a line element in shared memory, one pad element per 32: with an
-// odd line stride, the tile's loads (one element of each of 16 lines) and a
-// warp's reads along its line are free of bank conflicts
-__host__ __device__ constexpr int pad(int f) { return f + (f >> 5); }
 
 __host__ __device__ constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v >> 1); }
 __host__ __device__ constexpr int brev_c(int p, int bits) {
@@ -51,204 +45,155 @@ __host__ __device__ constexpr int brev_c(int p, int bits) {
   return r;
 }
 
-template <bool INV>
-__device__ __forceinline__ float2 twid(const float2* __restrict__ tw, int t) {
-  const float2 w = __ldg(tw + t);
-  return INV ? conjf2(w) : w;
+// cos and sin of 2 pi j / n (0 <= j <= n/2) at compile time: the Taylor
+// series of the angle folded into [0, pi/4]
+__host__ __device__ constexpr double taylor(double x, bool sine) {
+  double term = sine ? x : 1.0, sum = term;
+  for (int k = sine ? 2 : 1; k < 40; k += 2) {
+    term *= -x * x / (double)(k * (k + 1));
+    sum += term;
+  }
+  return sum;
+}
+__host__ __device__ constexpr double cos_turn(int j, int n);
+__host__ __device__ constexpr double sin_turn(int j, int n) {
+  return 4 * j > n ? sin_turn(n / 2 - j, n)
+                   : (8 * j > n ? taylor(6.283185307179586476925 * (n / 4 - j) / n, false)
+                                : taylor(6.283185307179586476925 * j / n, true));
+}
+__host__ __device__ constexpr double cos_turn(int j, int n) {
+  return 4 * j > n ? -cos_turn(n / 2 - j, n)
+                   : (8 * j > n ? taylor(6.283185307179586476925 * (n / 4 - j) / n, true)
+                                : taylor(6.283185307179586476925 * j / n, false));
 }
 
-// Per-lane twiddles of the 32-point stage across lanes, h = 16, 8, 4, 2:
-// W_(2h)^(lane mod h) on the lanes that take the difference (lane bit h
-// set), 1 on the others (forward sign).
-template <int N>
-__device__ __forceinline__ void lane_twiddles(const float2* __restrict__ tw, int lane, float2 (&wl)[4]) {
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const int h = 16 >> q;
-    const int t = (lane & (h - 1)) * (N / (2 * h));
-    wl[q] = (t == 0 || (lane & h) == 0) ? make_float2(1.f, 0.f) : __ldg(tw + t);
+// v W_M^j (INV: v W_M^-j) for constant j < M/2
+template <int M, int J, bool INV>
+__device__ __forceinline__ float2 turn(float2 v) {
+  if constexpr (J == 0) {
+    return v;
+  } else if constexpr (4 * J == M) {
+    return INV ? make_float2(-v.y, v.x) : make_float2(v.y, -v.x);
+  } else {
+    constexpr float c = (float)cos_turn(J, M), s = (float)sin_turn(J, M);
+    return cmul(v, make_float2(c, INV ? s : -s));
   }
 }
 
-// frequency held by lane l, register p after warp_fft<R>
-template <int R>
-__device__ __forceinline__ int freq_of(int lane, int p) {
-  return brev_c(p, ilog2(R)) + R * (int)(__brev((unsigned)lane) >> 27);
-}
-
-// Unnormalised DFT of an M = 32 R point line, sign -1 (INV: +1).
-// In: v[n1] = x[lane + 32 n1].  Out: v[p] = X[freq_of<R>(lane, p)].
-template <int N, int R, bool INV>
-__device__ __forceinline__ void warp_fft(float2 (&v)[R], int lane, const float2* __restrict__ tw,
-                                         const float2 (&wl)[4]) {
-  constexpr int M = 32 * R;
-  constexpr int S = N / M;
-  // R-point DIF over the registers
+// One stage of the register FFT: blocks of 2H, butterflies J, J + H.
+template <int R, int H, bool INV, int J>
+__device__ __forceinline__ void stage(float2 (&v)[R]) {
+  if constexpr (J < H) {
 #pragma unroll
-  for (int h = R / 2; h >= 1; h >>= 1) {
-#pragma unroll
-    for (int b = 0; b < R; b += 2 * h) {
-#pragma unroll
-      for (int j = 0; j < h; j++) {
-        const float2 a = v[b + j], c = v[b + j + h];
-        v[b + j] = cadd(a, c);
-        const float2 d = csub(a, c);
-        const int t = j * (N / (2 * h));
-        if (t == 0) v[b + j + h] = d;
-        else if (t == N / 4) v[b + j + h] = INV ? make_float2(-d.y, d.x) : make_float2(d.y, -d.x);
-        else v[b + j + h] = cmul(d, twid<INV>(tw, t));
+    for (int b = 0; b < R; b += 2 * H) {
+      const float2 a = v[b + J];
+      if (!INV) {
+        const float2 c = v[b + J + H];
+        v[b + J] = cadd(a, c);
+        v[b + J + H] = turn<2 * H, J, false>(csub(a, c));
+      } else {
+        const float2 c = turn<2 * H, J, true>(v[b + J + H]);
+        v[b + J] = cadd(a, c);
+        v[b + J + H] = csub(a, c);
       }
     }
-  }
-  // W_M^(lane k1), k1 = brev_R(p)
-#pragma unroll
-  for (int p = 1; p < R; p++) {
-    const int k1 = brev_c(p, ilog2(R));
-    v[p] = cmul(v[p], twid<INV>(tw, lane * k1 * S));
-  }
-  // 32-point DIF across the lanes: the lane of a pair with bit h clear keeps
-  // v + o, the other (o - v) W; one fused s v + o (s = +-1, exact) and one
-  // product with the lane's twiddle (1 on the first lane) serve both
-#pragma unroll
-  for (int q = 0; q < 5; q++) {
-    const int h = 16 >> q;
-    const float sg = (lane & h) ? -1.f : 1.f;
-#pragma unroll
-    for (int p = 0; p < R; p++) {
-      float2 o;
-      o.x = __shfl_xor_sync(FULL, v[p].x, h);
-      o.y = __shfl_xor_sync(FULL, v[p].y, h);
-      const float2 d = make_float2(__fmaf_rn(sg, v[p].x, o.x), __fmaf_rn(sg, v[p].y, o.y));
-      if (q < 4) v[p] = cmul(d, INV ? conjf2(wl[q]) : wl[q]);
-      else v[p] = d;
-    }
+    stage<R, H, INV, J + 1>(v);
   }
 }
 
-// z-pass tile: TY lines of NX values (padded), ZT threads
+// R-point DFT in registers, sign -1: natural order in, v[p] = X[brev(p)] out.
+template <int R, int H = R / 2>
+__device__ __forceinline__ void fft_reg(float2 (&v)[R]) {
+  if constexpr (H >= 1) {
+    stage<R, H, false, 0>(v);
+    fft_reg<R, H / 2>(v);
+  }
+}
+// The unnormalised inverse: v[p] = X[brev(p)] in, natural order out.
+template <int R, int H = 1>
+__device__ __forceinline__ void ifft_reg(float2 (&v)[R]) {
+  if constexpr (H < R) {
+    stage<R, H, true, 0>(v);
+    ifft_reg<R, 2 * H>(v);
+  }
+}
+
+// N = V T: V values a thread, T threads a line, 16 lines (128-byte runs of a
+// plane's rows) a CTA.  V and T near sqrt(N) keep the exchanges at one.
 template <int N>
 struct Geo {
-  static constexpr int NCOL = N / 2 + 1;         // kx = 0..N/2
-  static constexpr int LSTR = N + N / 32 + 1;    // line stride (float2): padded, odd
-  static constexpr int TY = 16;                  // lines per tile
-  static constexpr int ZT = 256;                 // threads
-  static constexpr size_t ZSMEM = sizeof(float2) * (size_t)TY * LSTR;
+  static constexpr int NCOL = N / 2 + 1;  // kx = 0..N/2
+  static constexpr int TY = 16;           // lines per tile
+  static constexpr int T = N >= 256 ? 16 : 8;
+  static constexpr int V = N / T;
+  static constexpr int ZT = TY * T;  // threads
+  static constexpr int MINB = N == 512 ? 3 : (N == 256 ? 4 : 8);  // CTAs an SM: 80 and 64 registers
+  static constexpr size_t ZSMEM = sizeof(float2) * (size_t)TY * N;
 };
 
 }  // namespace
-
-// The exact inverse of warp_fft<N, R, false> up to the factor M: the
-// unnormalised inverse DFT (sign +1) of a line held in warp_fft's output
-// order.  In: v[p] = X[freq_of<R>(lane, p)].  Out: v[n1] = x[lane + 32 n1].
-// Each stage undoes one of warp_fft's (decimation in time): across the lanes
-// the value of the lane with bit h set is first multiplied by its conjugate
-// twiddle, then the pair takes sum and difference.
-template <int N, int R>
-__device__ __forceinline__ void warp_ifft(float2 (&v)[R], int lane, const float2* __restrict__ tw,
-                                          const float2 (&wl)[4]) {
-  constexpr int M = 32 * R;
-  constexpr int S = N / M;
-#pragma unroll
-  for (int q = 4; q >= 0; q--) {
-    const int h = 16 >> q;
-    const float sg = (lane & h) ? -1.f : 1.f;
-#pragma unroll
-    for (int p = 0; p < R; p++) {
-      const float2 mm = q < 4 ? cmul(v[p], conjf2(wl[q])) : v[p];
-      float2 o;
-      o.x = __shfl_xor_sync(FULL, mm.x, h);
-      o.y = __shfl_xor_sync(FULL, mm.y, h);
-      v[p] = make_float2(__fmaf_rn(sg, mm.x, o.x), __fmaf_rn(sg, mm.y, o.y));
-    }
-  }
-#pragma unroll
-  for (int p = 1; p < R; p++) {
-    const int k1 = brev_c(p, ilog2(R));
-    v[p] = cmul(v[p], twid<true>(tw, lane * k1 * S));
-  }
-#pragma unroll
-  for (int h = 1; h <= R / 2; h <<= 1) {
-#pragma unroll
-    for (int b = 0; b < R; b += 2 * h) {
-#pragma unroll
-      for (int j = 0; j < h; j++) {
-        const float2 a = v[b + j], c = v[b + j + h];
-        const int t = j * (N / (2 * h));
-        float2 u;
-        if (t == 0) u = c;
-        else if (t == N / 4) u = make_float2(-c.y, c.x);  // c W^-1 = c i
-        else u = cmul(c, twid<true>(tw, t));
-        v[b + j] = cadd(a, u);
-        v[b + j + h] = csub(a, u);
-      }
-    }
-  }
-}
 
 // The z pass: a tile is TY consecutive values of one copy's (ky, kx) plane
 // ([copy][z][ky][kx], NX/2+1 values per row, as the library's 2-D R2C leaves
 // it), all NX z, in place: FFT along z, the Green's factor, inverse FFT
 // along z.  KKK / N^3 = (-DEL2 / N^3) x 1 / (s2[kx] + s2[ky] + s2[kz])
 // (denominator 1e30 at the origin; the reciprocal correctly rounded), on
-// both parts.  One warp per line; the tile moves through shared memory so
-// that every global access is a run of TY consecutive values.
+// both parts.  One read and one write of the spectrum: 1.08 GB in 0.25 ms at
+// 8 x 256^3 (0.65 of the measured copy rate) and in 0.32 ms at 512^3; with one
+// warp a line and the FFT across lanes by shuffles, 0.44 and 0.54 ms, held by
+// the shuffle queue.  What is left is the instruction issue of the two register
+// transforms.
 template <int N>
-__global__ void __launch_bounds__(Geo<N>::ZT)
+__global__ void __launch_bounds__(Geo<N>::ZT, Geo<N>::MINB)
 k_fft_z_green(float2* __restrict__ spec, const float2* __restrict__ tw, const float* __restrict__ s2,
               float del2, float inv_n3) {
   using G = Geo<N>;
-  constexpr int NW = G::ZT / 32, RZ = N / 32, QT = N * G::NCOL / G::TY;
-  constexpr int PER = G::TY * N / G::ZT;  // tile values per thread
-  extern __shared__ float2 sm[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int T = G::T, V = G::V, TY = G::TY, QT = N * G::NCOL / TY;
+  extern __shared__ float2 sm[];  // [k1][s][line]
+  const int j = threadIdx.x % TY, s = threadIdx.x / TY;
   const int64_t t = blockIdx.x;
-  const int q0 = (int)(t % QT) * G::TY;
-  const int64_t copy = t / QT;
+  const int qq = (int)(t % QT) * TY + j;
   const int64_t zstride = (int64_t)G::NCOL * N;
-  float2* base = spec + copy * N * zstride + q0;
+  float2* base = spec + (t / QT) * N * zstride + qq;
+  float2* own = sm + s * TY + j;
   {
-    float2 r[PER];
+    float2 v[V];
 #pragma unroll
-    for (int i = 0; i < PER; i++) {
-      const int e = threadIdx.x + G::ZT * i, z = e / G::TY, j = e % G::TY;
-      r[i] = base[z * zstride + j];
-    }
+    for (int n1 = 0; n1 < V; n1++) v[n1] = base[(int64_t)(s + T * n1) * zstride];
+    fft_reg<V>(v);
 #pragma unroll
-    for (int i = 0; i < PER; i++) {
-      const int e = threadIdx.x + G::ZT * i, z = e / G::TY, j = e % G::TY;
-      sm[j * G::LSTR + pad(z)] = r[i];
-    }
+    for (int p = 0; p < V; p++) own[brev_c(p, ilog2(V)) * T * TY] = v[p];
   }
   __syncthreads();
-  float2 wl[4];
-  lane_twiddles<N>(tw, lane, wl);
+  const int kx = qq % G::NCOL, ky = qq / G::NCOL;
   const float scale = __fmul_rn(-del2, inv_n3);
-  for (int q = warp; q < G::TY; q += NW) {
-    const int qq = q0 + q;
-    const int kx = qq % G::NCOL, ky = qq / G::NCOL;
-    float2* ln = sm + q * G::LSTR;
-    float2 v[RZ];
+  const float sxy = __fadd_rn(__ldg(s2 + kx), __ldg(s2 + ky));
 #pragma unroll
-    for (int n1 = 0; n1 < RZ; n1++) v[n1] = ln[pad(lane + 32 * n1)];
-    warp_fft<N, RZ, false>(v, lane, tw, wl);
-    const float sxy = __fadd_rn(__ldg(s2 + kx), __ldg(s2 + ky));
+  for (int g = 0; g < V / T; g++) {
+    const int k1 = s + T * g;
+    float2* row = sm + k1 * T * TY + j;
+    float2 u[T];
 #pragma unroll
-    for (int p = 0; p < RZ; p++) {
-      const int kz = freq_of<RZ>(lane, p);
+    for (int q = 0; q < T; q++) u[q] = cmul(row[q * TY], __ldg(tw + q * k1));
+    fft_reg<T>(u);
+#pragma unroll
+    for (int p = 0; p < T; p++) {
+      const int kz = k1 + V * brev_c(p, ilog2(T));
       const float den = (kx == 0 && ky == 0 && kz == 0) ? 1.0e30f : __fadd_rn(sxy, __ldg(s2 + kz));
       const float f = __fmul_rn(scale, __frcp_rn(den));
-      v[p] = make_float2(__fmul_rn(v[p].x, f), __fmul_rn(v[p].y, f));
+      u[p] = make_float2(__fmul_rn(u[p].x, f), __fmul_rn(u[p].y, f));
     }
-    warp_ifft<N, RZ>(v, lane, tw, wl);
+    ifft_reg<T>(u);
 #pragma unroll
-    for (int n1 = 0; n1 < RZ; n1++) ln[pad(lane + 32 * n1)] = v[n1];
+    for (int q = 0; q < T; q++) row[q * TY] = cmul(u[q], conjf2(__ldg(tw + q * k1)));
   }
   __syncthreads();
+  float2 v[V];
 #pragma unroll
-  for (int i = 0; i < PER; i++) {
-    const int e = threadIdx.x + G::ZT * i, z = e / G::TY, j = e % G::TY;
-    base[z * zstride + j] = sm[j * G::LSTR + pad(z)];
-  }
+  for (int p = 0; p < V; p++) v[p] = own[brev_c(p, ilog2(V)) * T * TY];
+  ifft_reg<V>(v);
+#pragma unroll
+  for (int n1 = 0; n1 < V; n1++) base[(int64_t)(s + T * n1) * zstride] = v[n1];
 }
 
 // W_N^j = exp(-2 pi i j / N), j < N, in double then rounded; exact at the
