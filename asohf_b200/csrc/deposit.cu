@@ -1793,12 +1793,13 @@ extern "C" int asohf_renorm_density(asohf_ctx* c, int nx, const asohf_mesh* mesh
 }
 
 // ------------------------------------------------------------ TSC deposit
-// Base grid TSC for a batch of particle sets (float32 sums, the layer's sizes
-// its sort does not cover).
+// Base grid TSC for a batch of particle sets in input order (the layer: float64
+// sums of its small sets, float32 at the sizes its sort does not cover).
+template <typename T>
 __global__ void k_tsc_base(const float* __restrict__ x, const float* __restrict__ y,
                            const float* __restrict__ z, const float* __restrict__ m, int64_t n_per,
                            int batch, int nx, float xl, float dx, const float* __restrict__ radx,
-                           float denbas, float* __restrict__ acc) {
+                           float denbas, T* __restrict__ acc) {
   int64_t ntot = n_per * batch;
   size_t g = (size_t)nx * nx * nx;
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < ntot;
@@ -1811,7 +1812,7 @@ __global__ void k_tsc_base(const float* __restrict__ x, const float* __restrict_
     tsc_weights(yp, radx[jy - 1], radx[jy], radx[jy + 1], dx, wy);
     tsc_weights(zp, radx[kz - 1], radx[kz], radx[kz + 1], dx, wz);
     float mp = denbas == 1.0f ? m[q] : __fdiv_rn(m[q], denbas);  // mass, or mass / DENBAS
-    float* a = acc + (size_t)b * g;
+    T* a = acc + (size_t)b * g;
 #pragma unroll
     for (int kk = -1; kk <= 1; kk++) {
       int k1 = kz + kk;
@@ -1828,7 +1829,7 @@ __global__ void k_tsc_base(const float* __restrict__ x, const float* __restrict_
           if (i1 == nx + 1) i1 = 1;
           if (i1 == 0) i1 = nx;
           float t = __fmul_rn(__fmul_rn(__fmul_rn(mp, wx[ii + 1]), wy[jj + 1]), wz[kk + 1]);
-          atomicAdd(&a[((size_t)(k1 - 1) * nx + (j1 - 1)) * nx + (i1 - 1)], t);
+          atomicAdd(&a[((size_t)(k1 - 1) * nx + (j1 - 1)) * nx + (i1 - 1)], (T)t);
         }
       }
     }
@@ -2162,12 +2163,30 @@ int tsc_base_batched_f32(asohf_ctx* c, int nx, float xl, float dx, const float* 
   if (n > 0) {
     {
       int kt_ = ktime_begin(c, "tsc_base_batched");
-      k_tsc_base<<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(x, y, z, m, n_per, batch,
+      k_tsc_base<float><<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(x, y, z, m, n_per, batch,
                                                                               nx, xl, dx, dradx, denbas, acc);
       ktime_end(c, kt_);
     }
     c->launches++;
   }
+  ASOHF_CUDA(cudaGetLastError());
+  return ASOHF_OK;
+}
+
+// the same in float64 sums (acc cleared by the caller), rounded into rho
+int tsc_base_batched_f64(asohf_ctx* c, int nx, float xl, float dx, const float* dradx, int batch,
+                         int64_t n_per, const float* x, const float* y, const float* z,
+                         const float* m, float denbas, double* acc, float* rho) {
+  const int64_t n = n_per * batch, g = (int64_t)nx * nx * nx * batch;
+  int kt_ = ktime_begin(c, "tsc_base_batched");
+  if (n > 0) {
+    k_tsc_base<double><<<grid_for(n, 128, c->num_sms * 16), 128, 0, c->stream>>>(x, y, z, m, n_per, batch, nx, xl, dx,
+                                                                             dradx, denbas, acc);
+    c->launches++;
+  }
+  k_finish_f64<<<grid_for(g, 256), 256, 0, c->stream>>>(acc, g, 1.0f, rho);
+  c->launches++;
+  ktime_end(c, kt_);
   ASOHF_CUDA(cudaGetLastError());
   return ASOHF_OK;
 }

@@ -25,6 +25,9 @@ int fftconv_z_green_2d(asohf_ctx* c, int nx, int batch, void* spec, const float*
 int tsc_base_batched_f32(asohf_ctx* c, int nx, float xl, float dx, const float* dradx, int batch,
                          int64_t n_per, const float* x, const float* y, const float* z,
                          const float* m, float denbas, float* acc);
+int tsc_base_batched_f64(asohf_ctx* c, int nx, float xl, float dx, const float* dradx, int batch,
+                         int64_t n_per, const float* x, const float* y, const float* z,
+                         const float* m, float denbas, double* acc, float* rho);
 
 #define ASOHF_CUFFT(call)                                                        \
   do {                                                                           \
@@ -102,25 +105,25 @@ static void momento_axis(int nx, float* s2) {
 }
 
 // Half-spectrum multiply: spec[(k*N + j)*(N/2+1) + i] *= KKK(i,j,k) / N^3.
-// A flat grid-stride loop over the complex values (consecutive threads take
-// consecutive values, so every warp access is one contiguous 256-byte run);
-// the (i, j, k) of a value come from its index, s2 from the L1-resident table.
-__global__ void k_green(cufftComplex* __restrict__ spec, int nx, int batch, const float* __restrict__ s2,
+// One warp a row (j, k): the row's indices are divided out once, the lanes take
+// consecutive values.  Bound by the two passes' memory at large sizes; 3 x 100^3
+// in 12.7 us (14.8 us with 64-bit divisions for every value).
+__global__ void k_green(cufftComplex* __restrict__ spec, int nx, int64_t rows, const float* __restrict__ s2,
                         float del2, float inv_n3) {
-  const int64_t nh = nx / 2 + 1;
-  const int64_t total = (int64_t)batch * nx * nx * nh;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-       q += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = q / nh;
-    const int i = (int)(q - row * nh), j = (int)(row % nx), k = (int)((row / nx) % nx);
-    const float den = (i == 0 && j == 0 && k == 0) ? 1.0e30f : __fadd_rn(__fadd_rn(__ldg(s2 + i), __ldg(s2 + j)),
-                                                                         __ldg(s2 + k));
-    const float kkk = -del2 / den;
-    const float f = __fmul_rn(kkk, inv_n3);
-    cufftComplex v = spec[q];
-    v.x = __fmul_rn(v.x, f);
-    v.y = __fmul_rn(v.y, f);
-    spec[q] = v;
+  const int nh = nx / 2 + 1, lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; row < rows; row += nw) {
+    const int j = (int)(row % nx), k = (int)((row / nx) % nx);
+    const float sj = __ldg(s2 + j), sk = __ldg(s2 + k);
+    cufftComplex* line = spec + row * nh;
+    for (int i = lane; i < nh; i += 32) {
+      const float den = (i == 0 && j == 0 && k == 0) ? 1.0e30f : __fadd_rn(__fadd_rn(__ldg(s2 + i), sj), sk);
+      const float f = __fmul_rn(-del2 / den, inv_n3);
+      cufftComplex v = line[i];
+      v.x = __fmul_rn(v.x, f);
+      v.y = __fmul_rn(v.y, f);
+      line[i] = v;
+    }
   }
 }
 
@@ -193,8 +196,8 @@ static int poisson_dev(asohf_ctx* c, int nx, float dx, int batch, const float* r
   ktime_end(c, kt_);
   {
     int kt_ = ktime_begin(c, "green_multiply");
-    const int64_t total = (int64_t)batch * nx * nx * (nx / 2 + 1);
-    k_green<<<grid_for(total, 256, c->num_sms * 16), 256, 0, c->stream>>>(spec, nx, batch, ds2, del2, inv_n3);
+    const int64_t rows = (int64_t)batch * nx * nx;
+    k_green<<<grid_for(32 * rows, 256, c->num_sms * 16), 256, 0, c->stream>>>(spec, nx, rows, ds2, del2, inv_n3);
     ktime_end(c, kt_);
   }
   c->launches++;
@@ -233,7 +236,7 @@ extern "C" int asohf_poisson_fft(asohf_ctx* c, int nx, float dx, int batch, cons
 }
 
 // ------------------------------------------------------------ layer
-// The layer's particles are sorted once per call by a key of (copy, Morton
+// The forward's particles are sorted once per call by a key of (copy, Morton
 // code of the host cell), so a warp reads 32 particles of neighbouring cells
 // and the grid cells it touches are close together.  Particles that share a
 // host cell share all 27 target cells: a warp adds each run of equal keys
@@ -253,6 +256,14 @@ __device__ __forceinline__ uint32_t spread3(uint32_t v) {
   v = (v | (v << 2)) & 0x09249249u;
   return v;
 }
+
+// Small sets deposit in input order into float64 sums, 27 atomics a particle,
+// rounded in one more pass: the launches of the sort cost more than the
+// atomics' contention (to about 180000 particles) and than clearing and
+// rounding the float64 grid (to 4M cells).  (In float32 the unsorted sums of a
+// crowded cell were up to five times further off than the sorted ones.)
+#define LAYER_SMALL_N (5 << 15)
+#define LAYER_SMALL_G (1 << 22)
 
 struct LayerSort {
   uint32_t* keys;  // sorted keys: copy << cbits | Morton(ix-1, jy-1, kz-1)
@@ -394,14 +405,6 @@ __global__ void __launch_bounds__(256) k_layer_deposit(const uint32_t* __restric
   }
 }
 
-// dL/dx_p = m_p/DENBAS * sum_c d(Wx Wy Wz)/dx_p * g_c,  g = G * w, over the
-// sorted particles (neighbouring warps read neighbouring cells of g).
-__global__ void k_layer_adjoint(const uint32_t* __restrict__ keys, const int32_t* __restrict__ idx,
-                                const float4* __restrict__ pm, int64_t ntot, int nx, int cbits, float xl,
-                                float dx, const float* __restrict__ radx, const float* __restrict__ gfield,
-                                float inv_denbas, float* __restrict__ gx, float* __restrict__ gy,
-                                float* __restrict__ gz, float* __restrict__ gm);
-
 extern "C" int asohf_tsc_poisson_forward(asohf_ctx* c, int nx, float lado0, float dx,
                                          const float* radx, float rote, float rete, int batch,
                                          int64_t n_per, const float* x, const float* y,
@@ -411,16 +414,23 @@ extern "C" int asohf_tsc_poisson_forward(asohf_ctx* c, int nx, float lado0, floa
   arena_reset(c);
   int64_t g = (int64_t)nx * nx * nx * batch;
   const int64_t ntot = n_per * batch;
-  const bool sorted = ntot > 0 && layer_sortable(nx, batch, ntot);
-  ASOHF_CHECK(arena_reserve(c, poisson_bytes(nx, batch) + (sorted ? layer_sort_bytes(nx, batch, ntot) : 0) + 1024));
+  const bool small = ntot <= LAYER_SMALL_N && g <= LAYER_SMALL_G;
+  const bool sorted = !small && layer_sortable(nx, batch, ntot);
+  ASOHF_CHECK(arena_reserve(c, poisson_bytes(nx, batch) + (sorted ? layer_sort_bytes(nx, batch, ntot) : 0) +
+                                   (small ? 8 * (size_t)g : 0) + 1024));
   const float* dradx;
   ASOHF_CHECK(radx_device(c, nx, radx, &dradx));
-  ASOHF_CUDA(cudaMemsetAsync(rho, 0, 4 * g, c->stream));
+  if (!small) ASOHF_CUDA(cudaMemsetAsync(rho, 0, 4 * g, c->stream));
   // each particle deposits m / (DX^3 ROTE RETE^3): the division of the cell
   // sums (grids.f:1236-1238) moved onto the terms, so rho needs no extra pass
   float denbas = dx * dx * dx * rote * (rete * rete * rete);
   const float xl = -lado0 / 2.0f;
-  if (sorted) {
+  if (small) {
+    double* acc = (double*)arena_alloc(c, 8 * (size_t)g);
+    if (!acc) return ASOHF_ERR_CAPACITY;
+    ASOHF_CUDA(cudaMemsetAsync(acc, 0, 8 * g, c->stream));
+    ASOHF_CHECK(tsc_base_batched_f64(c, nx, xl, dx, dradx, batch, n_per, x, y, z, m, denbas, acc, rho));
+  } else if (sorted) {
     LayerSort s;
     ASOHF_CHECK(layer_sort(c, nx, xl, dx, batch, n_per, x, y, z, m, &s));
     int kt_ = ktime_begin(c, "layer_deposit");
@@ -447,7 +457,11 @@ __device__ __forceinline__ void tsc_w_dw(float xp, float rm, float r0, float rp,
   w[2] = 0.5f * t * t; dw[2] = -t * copysignf(1.0f, s) / d;
 }
 
-// dL/dx_p = m_p/DENBAS * sum_c d(Wx Wy Wz)/dx_p * g_c,  g = G * w.
+// dL/dx_p = m_p/DENBAS * sum_c d(Wx Wy Wz)/dx_p * g_c,  g = G * w, particles in
+// input order.  The copies follow each other, so the cells in reach at a time
+// are about one copy's field, which the L2 holds to 256^3: 8 x 262144 particles
+// take 174 us on 256^3 and 128 us on 128^3, in cell order 172 and 135 us plus
+// 168 and 138 us for the keys and the sort.
 __global__ void k_tsc_adjoint(const float* __restrict__ x, const float* __restrict__ y,
                               const float* __restrict__ z, const float* __restrict__ m, int64_t n_per,
                               int batch, int nx, float xl, float dx, const float* __restrict__ radx,
@@ -500,54 +514,6 @@ __global__ void k_tsc_adjoint(const float* __restrict__ x, const float* __restri
   }
 }
 
-__global__ void k_layer_adjoint(const uint32_t* __restrict__ keys, const int32_t* __restrict__ idx,
-                                const float4* __restrict__ pm, int64_t ntot, int nx, int cbits, float xl,
-                                float dx, const float* __restrict__ radx, const float* __restrict__ gfield,
-                                float inv_denbas, float* __restrict__ gx, float* __restrict__ gy,
-                                float* __restrict__ gz, float* __restrict__ gm) {
-  const size_t G = (size_t)nx * nx * nx;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ntot;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t q = idx[i];
-    const float4 p = pm[q];
-    const int ix = tsc_cell(p.x, xl, dx, nx), jy = tsc_cell(p.y, xl, dx, nx), kz = tsc_cell(p.z, xl, dx, nx);
-    float wx[3], wy[3], wz[3], dwx[3], dwy[3], dwz[3];
-    tsc_w_dw(p.x, radx[ix - 1], radx[ix], radx[ix + 1], dx, wx, dwx);
-    tsc_w_dw(p.y, radx[jy - 1], radx[jy], radx[jy + 1], dx, wy, dwy);
-    tsc_w_dw(p.z, radx[kz - 1], radx[kz], radx[kz + 1], dx, wz, dwz);
-    const float* g = gfield + (size_t)(keys[i] >> cbits) * G;
-    float ax = 0.f, ay = 0.f, az = 0.f, am = 0.f;
-#pragma unroll
-    for (int kk = -1; kk <= 1; kk++) {
-      int k1 = kz + kk;
-      if (k1 == nx + 1) k1 = 1;
-      if (k1 == 0) k1 = nx;
-#pragma unroll
-      for (int jj = -1; jj <= 1; jj++) {
-        int j1 = jy + jj;
-        if (j1 == nx + 1) j1 = 1;
-        if (j1 == 0) j1 = nx;
-#pragma unroll
-        for (int ii = -1; ii <= 1; ii++) {
-          int i1 = ix + ii;
-          if (i1 == nx + 1) i1 = 1;
-          if (i1 == 0) i1 = nx;
-          float gv = g[((size_t)(k1 - 1) * nx + (j1 - 1)) * nx + (i1 - 1)];
-          ax += dwx[ii + 1] * wy[jj + 1] * wz[kk + 1] * gv;
-          ay += wx[ii + 1] * dwy[jj + 1] * wz[kk + 1] * gv;
-          az += wx[ii + 1] * wy[jj + 1] * dwz[kk + 1] * gv;
-          am += wx[ii + 1] * wy[jj + 1] * wz[kk + 1] * gv;
-        }
-      }
-    }
-    const float mp = p.w * inv_denbas;
-    gx[q] = mp * ax;
-    gy[q] = mp * ay;
-    gz[q] = mp * az;
-    if (gm) gm[q] = am * inv_denbas;
-  }
-}
-
 extern "C" int asohf_tsc_poisson_adjoint(asohf_ctx* c, int nx, float lado0, float dx,
                                          const float* radx, float rote, float rete, int batch,
                                          int64_t n_per, const float* x, const float* y,
@@ -558,26 +524,15 @@ extern "C" int asohf_tsc_poisson_adjoint(asohf_ctx* c, int nx, float lado0, floa
   arena_reset(c);
   int64_t g = (int64_t)nx * nx * nx * batch;
   int64_t ntot = n_per * batch;
-  const bool sorted = ntot > 0 && layer_sortable(nx, batch, ntot);
-  ASOHF_CHECK(arena_reserve(c, poisson_bytes(nx, batch) + 4 * g + (sorted ? layer_sort_bytes(nx, batch, ntot) : 0) +
-                                   2048));
+  ASOHF_CHECK(arena_reserve(c, poisson_bytes(nx, batch) + 4 * g + 2048));
   const float* dradx;
   ASOHF_CHECK(radx_device(c, nx, radx, &dradx));
   float* gfield = (float*)arena_alloc(c, 4 * g);
   if (!gfield) return ASOHF_ERR_CAPACITY;
   float denbas = dx * dx * dx * rote * (rete * rete * rete);
-  const float xl = -lado0 / 2.0f;
-  LayerSort s;
-  if (sorted) ASOHF_CHECK(layer_sort(c, nx, xl, dx, batch, n_per, x, y, z, m, &s));
   // the Green's operator is real and symmetric: its adjoint is itself
   ASOHF_CHECK(poisson_dev(c, nx, dx, batch, w, gfield));
-  if (sorted) {
-    int kt_ = ktime_begin(c, "layer_adjoint");
-    k_layer_adjoint<<<grid_for(ntot, 256, c->num_sms * 16), 256, 0, c->stream>>>(
-        s.keys, s.idx, s.pm, ntot, nx, s.cbits, xl, dx, dradx, gfield, 1.0f / denbas, grad_x, grad_y, grad_z, grad_m);
-    ktime_end(c, kt_);
-    c->launches++;
-  } else if (ntot > 0) {
+  if (ntot > 0) {
     {
       int kt_ = ktime_begin(c, "tsc_adjoint_gather");
       k_tsc_adjoint<<<grid_for(ntot, 256, c->num_sms * 16), 256, 0, c->stream>>>(
