@@ -428,27 +428,49 @@ int clean_in(asohf_ctx* c, const asohf_catalogue* cat, int n, int on_device, Cle
   io->h_rc = cat->realclus;
   ASOHF_CHECK(arena_reserve(c, (on_device ? 0 : (size_t)n * 40 + 10 * 256) + x_order_bytes(n) + 4096));
   if (on_device) {
+    ASOHF_CHECK(hst_reserve(c, 1024));
     io->d = CleanCat{cat->clusrx, cat->clusry, cat->clusrz, speeds ? cat->vx : nullptr, speeds ? cat->vy : nullptr,
                      speeds ? cat->vz : nullptr, speeds ? cat->masa : nullptr, cat->radio, cat->levhal, cat->realclus};
     return ASOHF_OK;
   }
-  const float* hf[8] = {cat->clusrx, cat->clusry, cat->clusrz, cat->vx, cat->vy, cat->vz, cat->masa, cat->radio};
-  float* df[8];
-  for (int q = 0; q < 8; q++) {
+  // one block through page-locked staging: up to 8 fields, levels, REALCLUS
+  const void* hf[10] = {cat->clusrx, cat->clusry, cat->clusrz, cat->vx, cat->vy, cat->vz, cat->masa, cat->radio,
+                        cat->levhal, cat->realclus};
+  const size_t row = (4 * (size_t)n + 15) & ~(size_t)15;
+  ASOHF_CHECK(hst_reserve(c, 11 * row + 1024));
+  char* hb = (char*)hst_alloc(c, 10 * row + 16);
+  char* db = (char*)arena_alloc(c, 10 * row + 16);
+  if (!hb || !db) return ASOHF_ERR_CAPACITY;
+  char* df[10];
+  size_t at = 0;
+  for (int q = 0; q < 10; q++) {
     df[q] = nullptr;
     if (!speeds && q >= 3 && q <= 6) continue;
-    df[q] = (float*)arena_alloc(c, 4 * (size_t)n + 4);
-    if (!df[q]) return ASOHF_ERR_CAPACITY;
-    if (n) ASOHF_CUDA(cudaMemcpyAsync(df[q], hf[q], 4 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
+    df[q] = db + at;
+    memcpy(hb + at, hf[q], 4 * (size_t)n);
+    at += row;
   }
-  int32_t* dl = (int32_t*)arena_alloc(c, 4 * (size_t)n + 4);
-  int32_t* dr = (int32_t*)arena_alloc(c, 4 * (size_t)n + 4);
-  if (!dl || !dr) return ASOHF_ERR_CAPACITY;
-  if (n) {
-    ASOHF_CUDA(cudaMemcpyAsync(dl, cat->levhal, 4 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
-    ASOHF_CUDA(cudaMemcpyAsync(dr, cat->realclus, 4 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
-  }
-  io->d = CleanCat{df[0], df[1], df[2], df[3], df[4], df[5], df[6], df[7], dl, dr};
+  if (n) ASOHF_CUDA(cudaMemcpyAsync(db, hb, at, cudaMemcpyHostToDevice, c->stream));
+  auto f = [&](int q) { return (const float*)df[q]; };
+  io->d = CleanCat{f(0), f(1), f(2), f(3), f(4), f(5), f(6), f(7), (const int32_t*)df[8], (int32_t*)df[9]};
+  return ASOHF_OK;
+}
+
+// REALCLUS of entries a..b-1 (a host catalogue) and `nw` words of device
+// results, staged; returns with the stream idle.  The caller copies the
+// entries from *rc when it accepts the results.
+int clean_out(asohf_ctx* c, const CleanIo& io, int a, int b, const int* dwords, int nw, int* hwords,
+              const int32_t** rc) {
+  int* w = (int*)hst_alloc(c, 4 * (size_t)nw);
+  int32_t* h = io.host ? (int32_t*)hst_alloc(c, 4 * (size_t)(b - a)) : nullptr;
+  if (!w || (io.host && !h)) return ASOHF_ERR_CAPACITY;
+  ASOHF_CUDA(cudaMemcpyAsync(w, dwords, 4 * (size_t)nw, cudaMemcpyDeviceToHost, c->stream));
+  if (io.host && b > a)
+    ASOHF_CUDA(cudaMemcpyAsync(h, io.d.rc + a, 4 * (size_t)(b - a), cudaMemcpyDeviceToHost, c->stream));
+  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  c->hst_busy = false;
+  memcpy(hwords, w, 4 * (size_t)nw);
+  *rc = h;
   return ASOHF_OK;
 }
 
@@ -502,13 +524,10 @@ extern "C" int asohf_check_rubish(asohf_ctx* c, asohf_catalogue* cat, int nclus,
   ktime_end(c, kt_);
   ASOHF_CUDA(cudaGetLastError());
   int hflags[2];
-  ASOHF_CUDA(cudaMemcpyAsync(hflags, dflags, 8, cudaMemcpyDeviceToHost, c->stream));
-  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  const int32_t* hrc;
+  ASOHF_CHECK(clean_out(c, io, low1 - 1, low2, dflags, 2, hflags, &hrc));
   if (hflags[0]) return ASOHF_ERR_UNSUPPORTED;  // a live pair with a zero speed (see the top of the file)
-  if (io.host && low2 >= low1)
-    ASOHF_CUDA(cudaMemcpyAsync(cat->realclus + low1 - 1, io.d.rc + low1 - 1, 4 * (size_t)(low2 - low1 + 1),
-                               cudaMemcpyDeviceToHost, c->stream));
-  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  if (io.host) memcpy(cat->realclus + low1 - 1, hrc, 4 * (size_t)(low2 - low1 + 1));
   if (removed) *removed = hflags[1];
   return ASOHF_OK;
 }
@@ -550,10 +569,9 @@ extern "C" int asohf_accidental_substructure(asohf_ctx* c, asohf_catalogue* cat,
   ktime_end(c, kt_);
   ASOHF_CUDA(cudaGetLastError());
   int hcount = 0;
-  ASOHF_CUDA(cudaMemcpyAsync(&hcount, dcount, 4, cudaMemcpyDeviceToHost, c->stream));
-  if (io.host)
-    ASOHF_CUDA(cudaMemcpyAsync(cat->realclus, io.d.rc, 4 * (size_t)nclus, cudaMemcpyDeviceToHost, c->stream));
-  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  const int32_t* hrc;
+  ASOHF_CHECK(clean_out(c, io, 0, nclus, dcount, 1, &hcount, &hrc));
+  if (io.host) memcpy(cat->realclus, hrc, 4 * (size_t)nclus);
   if (removed) *removed = hcount;
   return ASOHF_OK;
 }

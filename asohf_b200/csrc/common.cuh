@@ -122,6 +122,12 @@ struct asohf_ctx {
   // kernel phases of one call, when the stream is idle
   char* seg = nullptr;
   size_t seg_size = 0, seg_used = 0;
+  // page-locked staging for the small host arrays of one call (bump
+  // allocator, reset by hst_reserve at its start; every call that uses it ends
+  // with its copies done)
+  char* hst = nullptr;
+  size_t hst_size = 0, hst_used = 0;
+  bool hst_busy = false;  // copies from or to it may be in flight
   // Deferred patch deposit (asohf_set_density_overlap): with device outputs
   // the patch kernels of asohf_density (and RENORM_DENSITY's patch scaling)
   // run on dens_stream from the two density pools, which later calls do not
@@ -181,6 +187,11 @@ void* dpool_alloc(asohf_ctx* c, int which, size_t bytes);
 // Waits (host) for a deferred patch deposit still in flight.
 int density_settle(asohf_ctx* c);
 void* seg_alloc(asohf_ctx* c, size_t bytes);
+
+// Page-locked staging: hst_reserve starts a call's use (contents lost), after
+// waiting for a use that did not clear hst_busy at its end.
+int hst_reserve(asohf_ctx* c, size_t bytes);
+void* hst_alloc(asohf_ctx* c, size_t bytes);  // 64-byte aligned, nullptr if full
 
 int ctx_ensure_particles(asohf_ctx* c, int64_t n);
 void ctx_swap_particles(asohf_ctx* c);

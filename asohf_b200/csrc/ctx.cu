@@ -170,6 +170,28 @@ void* seg_alloc(asohf_ctx* c, size_t bytes) {
   return p;
 }
 
+int hst_reserve(asohf_ctx* c, size_t bytes) {
+  c->hst_used = 0;
+  if (c->hst_busy) ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  c->hst_busy = true;
+  if (c->hst_size >= bytes) return ASOHF_OK;
+  cudaFreeHost(c->hst);
+  c->hst = nullptr;
+  c->hst_size = 0;
+  const size_t want = bytes + bytes / 2;
+  ASOHF_CUDA(cudaMallocHost(&c->hst, want));
+  c->hst_size = want;
+  return ASOHF_OK;
+}
+
+void* hst_alloc(asohf_ctx* c, size_t bytes) {
+  const size_t b = (bytes + 63) & ~(size_t)63;
+  if (c->hst_used + b > c->hst_size) return nullptr;
+  void* p = c->hst + c->hst_used;
+  c->hst_used += b;
+  return p;
+}
+
 __global__ void k_minmax(const float* __restrict__ m, int64_t n, float* out) {
   __shared__ float sb[32];
   float lo = INFINITY, hi = -INFINITY;
@@ -279,6 +301,7 @@ extern "C" int asohf_destroy(asohf_ctx* c) {
   cudaFree(c->sfin_v);
   cudaFree(c->arena);
   cudaFree(c->seg);
+  cudaFreeHost(c->hst);
   cudaFree(c->d_work);
   for (int i = 0; i < asohf_ctx::NSIDE; i++) {
     cudaStreamSynchronize(c->side[i]);

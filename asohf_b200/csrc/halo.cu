@@ -33,8 +33,11 @@
 // ---------------------------------------------------------------- catalogue mirror
 // A call reads and writes the entries of its own haloes, [w0, n), and (the
 // subhalo calls) a few fields of earlier entries, their hosts.  With a host
-// catalogue only those ranges cross PCIe; the device arrays keep the
-// caller's indexing.
+// catalogue only those ranges cross PCIe, all fields of a call packed in
+// page-locked staging and moved as one block each way; the device pointers are
+// shifted so that the kernels keep the caller's indexing.  (A copy a field, 45
+// each way, took 1.0 ms of a call's 1.4 ms on the host at a few hundred
+// haloes.)  INDCS is host work and stays there.
 struct CatMirror {
   asohf_catalogue h;  // caller's
   asohf_catalogue d;  // device
@@ -42,6 +45,8 @@ struct CatMirror {
   int w0;             // first entry of the call's window
   bool host;
   bool prune;         // only the fields PRUNE_POOR_HALOES reads and writes move
+  char *hblk, *dblk;  // the packed window fields, staged and on the device
+  size_t bytes;
 };
 
 #define CAT_F1(X) X(masa) X(radio) X(clusrx) X(clusry) X(clusrz) X(clusrxcm) X(clusrycm) X(clusrzcm) \
@@ -50,9 +55,8 @@ struct CatMirror {
   X(m2500m) X(r2500m) X(velocity_dispersion) X(kinetic_e) X(potential_e)
 #define CAT_I1(X) X(patchclus) X(realclus) X(levhal) X(dmpclus) X(iplip)
 #define CAT_FM(X) X(angularm, 3) X(profiles, 2 * ASOHF_NBINS) X(eigenval, 3) X(inertia_tensor, 6)
-// fields PRUNE_POOR_HALOES reads, and writes
+// fields PRUNE_POOR_HALOES reads; it writes the last two
 #define CAT_PRUNE_IN(X) X(clusrx) X(clusry) X(clusrz) X(radio) X(realclus) X(dmpclus)
-#define CAT_PRUNE_OUT(X) X(realclus) X(dmpclus)
 // fields of host entries the subhalo kernels read
 #define CAT_HOST(X) X(realclus, 1) X(masa, 1) X(msub, 1) X(clusrx, 1) X(clusry, 1) X(clusrz, 1) \
   X(profiles, 2 * ASOHF_NBINS)
@@ -69,6 +73,20 @@ static size_t cat_bytes(int n) {
   return b;
 }
 
+// Whether a subhalo call reads the field of host entries (its rows start at 0).
+#define CAT_IS_HOST(f, w) || !strcmp(name, #f)
+static bool cat_host_field(const char* name) { return false CAT_HOST(CAT_IS_HOST); }
+
+// Offset of the next packed field of `rows` rows of w words.
+static size_t cat_next(size_t* at, size_t rows, int w) {
+  const size_t o = *at;
+  *at += (4 * rows * (size_t)w + 15) & ~(size_t)15;
+  return o;
+}
+
+// Staging a call needs for the mirror of n entries.
+static size_t cat_stage_bytes(int n) { return 2 * cat_bytes(n); }
+
 static int cat_mirror_in(asohf_ctx* c, asohf_catalogue* h, int n, int on_device, CatMirror* m, int w0,
                          bool hosts = false, bool prune = false) {
   m->h = *h;
@@ -76,61 +94,86 @@ static int cat_mirror_in(asohf_ctx* c, asohf_catalogue* h, int n, int on_device,
   m->w0 = w0 < 0 ? 0 : (w0 > n ? n : w0);
   m->host = !on_device;
   m->prune = prune;
-  if (on_device) { m->d = *h; return ASOHF_OK; }
+  m->hblk = m->dblk = nullptr;
+  m->bytes = 0;
   m->d = *h;
+  if (on_device) return ASOHF_OK;
   const size_t a = (size_t)m->w0, cnt = (size_t)(n - m->w0);
-  if (prune) {  // the prune kernels touch six fields of the window
-#define P(f)                                                                                        \
-  m->d.f = (decltype(m->d.f))arena_alloc(c, 4 * (size_t)n + 4);                                    \
-  if (!m->d.f) return ASOHF_ERR_CAPACITY;                                                           \
-  if (cnt) ASOHF_CUDA(cudaMemcpyAsync(m->d.f + a, h->f + a, 4 * cnt, cudaMemcpyHostToDevice, c->stream));
-    CAT_PRUNE_IN(P)
-#undef P
-    return ASOHF_OK;
+  // fields of the window first, in one block; the hosts' fields after it
+  size_t total = 0, hat = 0;
+#define SZ(f, w) if (!(hosts && cat_host_field(#f))) cat_next(&total, cnt, w);
+#define SZ1(f) SZ(f, 1)
+#define HZ(f, w) cat_next(&hat, (size_t)n, w);
+  if (prune) { CAT_PRUNE_IN(SZ1) }
+  else { CAT_F1(SZ1) CAT_I1(SZ1) CAT_FM(SZ) }
+  if (hosts) { CAT_HOST(HZ) }
+#undef SZ
+#undef SZ1
+#undef HZ
+  m->hblk = (char*)hst_alloc(c, total + hat + 16);
+  m->dblk = (char*)arena_alloc(c, total + hat + 16);
+  if (!m->hblk || !m->dblk) return ASOHF_ERR_CAPACITY;
+  m->bytes = total;
+  size_t at = 0;
+#define F(f, w)                                                                      \
+  if (!(hosts && cat_host_field(#f))) {                                              \
+    const size_t o = cat_next(&at, cnt, w);                                          \
+    memcpy(m->hblk + o, h->f + a * (w), 4 * cnt * (w));                              \
+    m->d.f = (decltype(m->d.f))((uintptr_t)(m->dblk + o) - 4 * a * (w));             \
   }
-#define F(f)                                                                                        \
-  m->d.f = (decltype(m->d.f))arena_alloc(c, 4 * (size_t)n + 4);                                    \
-  if (!m->d.f) return ASOHF_ERR_CAPACITY;                                                           \
-  if (cnt) ASOHF_CUDA(cudaMemcpyAsync(m->d.f + a, h->f + a, 4 * cnt, cudaMemcpyHostToDevice, c->stream));
-  CAT_F1(F) CAT_I1(F)
+#define F1(f) F(f, 1)
+#define HF(f, w)                                                                     \
+  {                                                                                  \
+    const size_t o = cat_next(&at, (size_t)n, w);                                    \
+    memcpy(m->hblk + o, h->f, 4 * (size_t)n * (w));                                  \
+    m->d.f = (decltype(m->d.f))(m->dblk + o);                                        \
+  }
+  if (prune) { CAT_PRUNE_IN(F1) }
+  else { CAT_F1(F1) CAT_I1(F1) CAT_FM(F) }
+  if (hosts) { CAT_HOST(HF) }
 #undef F
-#define M(f, w)                                                                                     \
-  m->d.f = (float*)arena_alloc(c, 4 * (size_t)n * (w) + 4);                                        \
-  if (!m->d.f) return ASOHF_ERR_CAPACITY;                                                           \
-  if (cnt) ASOHF_CUDA(cudaMemcpyAsync(m->d.f + a * (w), h->f + a * (w), 4 * cnt * (w), cudaMemcpyHostToDevice, \
-                                      c->stream));
-  CAT_FM(M)
-#undef M
-  m->d.indcs = (int32_t*)arena_alloc(c, 8 * (size_t)n + 8);
-  if (!m->d.indcs) return ASOHF_ERR_CAPACITY;
-  if (cnt) ASOHF_CUDA(cudaMemcpyAsync(m->d.indcs + 2 * a, h->indcs + 2 * a, 8 * cnt, cudaMemcpyHostToDevice, c->stream));
-  if (hosts && a) {
-#define H(f, w) ASOHF_CUDA(cudaMemcpyAsync(m->d.f, h->f, 4 * a * (w), cudaMemcpyHostToDevice, c->stream));
-    CAT_HOST(H)
-#undef H
-  }
+#undef F1
+#undef HF
+  m->d.indcs = nullptr;
+  if (total + hat) ASOHF_CUDA(cudaMemcpyAsync(m->dblk, m->hblk, total + hat, cudaMemcpyHostToDevice, c->stream));
   return ASOHF_OK;
 }
 
-static int cat_mirror_out(asohf_ctx* c, CatMirror* m) {
-  if (!m->host || m->n == m->w0) return ASOHF_OK;
-  const size_t a = (size_t)m->w0, cnt = (size_t)(m->n - m->w0);
-  if (m->prune) {
-#define P(f) ASOHF_CUDA(cudaMemcpyAsync(m->h.f + a, m->d.f + a, 4 * cnt, cudaMemcpyDeviceToHost, c->stream));
-    CAT_PRUNE_OUT(P)
-#undef P
+// The window back to the caller; returns with the stream idle.
+static int cat_mirror_out(asohf_ctx* c, CatMirror* m, bool hosts = false) {
+  if (!m->host || m->n == m->w0) {
     ASOHF_CUDA(cudaStreamSynchronize(c->stream));
     return ASOHF_OK;
   }
-#define F(f) ASOHF_CUDA(cudaMemcpyAsync(m->h.f + a, m->d.f + a, 4 * cnt, cudaMemcpyDeviceToHost, c->stream));
-  CAT_F1(F) CAT_I1(F)
-#undef F
-#define M(f, w) \
-  ASOHF_CUDA(cudaMemcpyAsync(m->h.f + a * (w), m->d.f + a * (w), 4 * cnt * (w), cudaMemcpyDeviceToHost, c->stream));
-  CAT_FM(M)
-#undef M
-  ASOHF_CUDA(cudaMemcpyAsync(m->h.indcs + 2 * a, m->d.indcs + 2 * a, 8 * cnt, cudaMemcpyDeviceToHost, c->stream));
+  const size_t a = (size_t)m->w0, cnt = (size_t)(m->n - m->w0);
+  if (m->prune) {  // the two last fields of the block
+    const size_t f = (4 * cnt + 15) & ~(size_t)15;
+    char* b = m->hblk + m->bytes - 2 * f;
+    ASOHF_CUDA(cudaMemcpyAsync(b, m->dblk + m->bytes - 2 * f, 2 * f, cudaMemcpyDeviceToHost, c->stream));
+    ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+    c->hst_busy = false;
+    memcpy(m->h.realclus + a, b, 4 * cnt);
+    memcpy(m->h.dmpclus + a, b + f, 4 * cnt);
+    return ASOHF_OK;
+  }
+  ASOHF_CUDA(cudaMemcpyAsync(m->hblk, m->dblk, m->bytes, cudaMemcpyDeviceToHost, c->stream));
+  if (hosts) {  // the window part of the hosts' fields, into their place in the staging
+#define HF(f, w)                                                                                       \
+  {                                                                                                    \
+    const size_t o = (size_t)((char*)m->d.f - m->dblk) + 4 * a * (w);                                  \
+    ASOHF_CUDA(cudaMemcpyAsync(m->hblk + o, m->dblk + o, 4 * cnt * (w), cudaMemcpyDeviceToHost, c->stream)); \
+  }
+    CAT_HOST(HF)
+#undef HF
+  }
   ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  c->hst_busy = false;
+#define F(f, w) \
+  memcpy(m->h.f + a * (w), m->hblk + ((char*)(m->d.f + a * (w)) - m->dblk), 4 * cnt * (w));
+#define F1(f) F(f, 1)
+  CAT_F1(F1) CAT_I1(F1) CAT_FM(F)
+#undef F
+#undef F1
   return ASOHF_OK;
 }
 
@@ -227,6 +270,7 @@ extern "C" int asohf_prune_poor_haloes(asohf_ctx* c, const asohf_consts* k, asoh
   double ht = htime_now();
   arena_reset(c);
   ASOHF_CHECK(arena_reserve(c, cat_bytes(low2) + 4096));
+  if (!on_device) ASOHF_CHECK(hst_reserve(c, 32 * (size_t)(low2 - low1 + 1) + 4096));
   CatMirror m;
   ASOHF_CHECK(cat_mirror_in(c, cat, low2, on_device, &m, low1 - 1, false, true));
   int nh = low2 - low1 + 1;
@@ -241,7 +285,6 @@ extern "C" int asohf_prune_poor_haloes(asohf_ctx* c, const asohf_consts* k, asoh
   c->launches++;
   ASOHF_CUDA(cudaGetLastError());
   ASOHF_CHECK(cat_mirror_out(c, &m));
-  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
   htime_end(c, "host:prune", ht);
   return ASOHF_OK;
 }
@@ -304,8 +347,13 @@ struct Tiers {
 // slot ids[i] (slot i when ids is null).  dbuf holds n entries.
 static int split_tiers(asohf_ctx* c, const int32_t* hcount, int n, int32_t* dbuf, Tiers* T,
                        const int32_t* ids = nullptr) {
-  std::vector<int32_t> h_v((size_t)(n > 0 ? n : 1));
-  int32_t* h = h_v.data();
+  std::vector<int32_t> h_v;
+  int32_t* h = (int32_t*)hst_alloc(c, 4 * (size_t)n);
+  const bool staged = h != nullptr;  // else pageable: waited for
+  if (!staged) {
+    h_v.resize((size_t)(n > 0 ? n : 1));
+    h = h_v.data();
+  }
   int cnt[4] = {0, 0, 0, 0};
   auto tier = [&](int32_t k) {
     return k >= c->cluster_min ? 3 : (k >= c->tier2_k ? 2 : (k >= c->tier1_k ? 1 : 0));
@@ -319,7 +367,7 @@ static int split_tiers(asohf_ctx* c, const int32_t* hcount, int n, int32_t* dbuf
   int fill[4] = {off[0], off[1], off[2], off[3]};
   for (int i = 0; i < n; i++) h[fill[tier(hcount[i])]++] = ids ? ids[i] : i;
   if (n) ASOHF_CUDA(cudaMemcpyAsync(dbuf, h, 4 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
-  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  if (!staged) ASOHF_CUDA(cudaStreamSynchronize(c->stream));
   for (int t = 0; t < 4; t++) {
     T->n[t] = cnt[t];
     T->slots[t] = dbuf + off[t];
@@ -338,8 +386,13 @@ static int split_cluster_tier(asohf_ctx* c, const int32_t* hcount, int n, int cb
     if (cb < 16) return k > 4 * sh ? 0 : 2;  // 8 CTAs at most
     return k > 8 * sh ? 0 : (k > 4 * sh ? 1 : 2);
   };
-  std::vector<int32_t> h_v((size_t)(T->n[3] > 0 ? T->n[3] : 1));
-  int32_t* h = h_v.data();
+  std::vector<int32_t> h_v;
+  int32_t* h = (int32_t*)hst_alloc(c, 4 * (size_t)T->n[3]);
+  const bool staged = h != nullptr;
+  if (!staged) {
+    h_v.resize((size_t)(T->n[3] > 0 ? T->n[3] : 1));
+    h = h_v.data();
+  }
   int cnt[3] = {0, 0, 0};
   for (int i = 0; i < n; i++)
     if (hcount[i] >= c->cluster_min) cnt[pick(hcount[i])]++;
@@ -347,7 +400,7 @@ static int split_cluster_tier(asohf_ctx* c, const int32_t* hcount, int n, int cb
   for (int i = 0; i < n; i++)
     if (hcount[i] >= c->cluster_min) h[fill[pick(hcount[i])]++] = i;
   if (T->n[3]) ASOHF_CUDA(cudaMemcpyAsync(T->slots[3], h, 4 * (size_t)T->n[3], cudaMemcpyHostToDevice, c->stream));
-  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  if (!staged) ASOHF_CUDA(cudaStreamSynchronize(c->stream));
   for (int q = 0; q < 3; q++) {
     nsub[q] = cnt[q];
     sub[q] = T->slots[3] + (q == 0 ? 0 : (q == 1 ? cnt[0] : cnt[0] + cnt[1]));
@@ -1932,59 +1985,56 @@ int ensure_pph(asohf_ctx* c, int64_t need) {
 }
 
 // Host part of the ID concatenation (haloes_particles.f:1377-1408): INDCS of
-// haloes low1..low2 from the counts, offsets for k_write_ids.
+// haloes low1..low2 from the counts, offsets for k_write_ids.  A host
+// catalogue's INDCS is written in place; d_ids_off is enqueued from staging.
 int assign_id_offsets(asohf_ctx* c, CatMirror& m, int low1, int low2, const int32_t* work, int nslots,
                       const int32_t* d_nbound, int64_t* d_ids_off, int64_t* total_out) {
-  int n = low2;
-  std::vector<int32_t> realclus_v((size_t)n);
-  int32_t* realclus = realclus_v.data();
-  std::vector<int32_t> indcs_v(2 * (size_t)n);
-  int32_t* indcs = indcs_v.data();
-  std::vector<int32_t> nbound_v((size_t)(nslots > 0 ? nslots : 1));
-  int32_t* nbound = nbound_v.data();
-  std::vector<int64_t> ids_off_v((size_t)(nslots > 0 ? nslots : 1));
-  int64_t* ids_off = ids_off_v.data();
-  std::vector<int32_t> slot_of_v((size_t)(low2 - low1 + 1));
-  int32_t* slot_of = slot_of_v.data();
-  // entries before the window: from the caller's arrays when they are on the host
-  int h0 = m.host ? m.w0 : 0;
-  if (h0) {
-    memcpy(realclus, m.h.realclus, 4 * (size_t)h0);
-    memcpy(indcs, m.h.indcs, 8 * (size_t)h0);
+  const int n = low2, nw = low2 - low1 + 1;
+  // entries before the window come from the caller's arrays when on the host
+  const int h0 = m.host ? low1 - 1 : 0;
+  std::vector<int32_t> ind_v;
+  int32_t* realclus = (int32_t*)hst_alloc(c, 4 * (size_t)(n - h0));  // entries h0..n-1
+  int32_t* nbound = (int32_t*)hst_alloc(c, 4 * (size_t)nslots);
+  int64_t* ids_off = (int64_t*)hst_alloc(c, 8 * (size_t)nslots);
+  if (!realclus || !nbound || !ids_off) return ASOHF_ERR_CAPACITY;
+  int32_t* indcs = m.h.indcs;
+  ASOHF_CUDA(cudaMemcpyAsync(realclus, m.d.realclus + h0, 4 * (size_t)(n - h0), cudaMemcpyDeviceToHost, c->stream));
+  if (!m.host) {
+    ind_v.resize(2 * (size_t)n);
+    indcs = ind_v.data();
+    ASOHF_CUDA(cudaMemcpyAsync(indcs, m.d.indcs, 8 * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
   }
-  ASOHF_CUDA(cudaMemcpyAsync(realclus + h0, m.d.realclus + h0, 4 * (size_t)(n - h0), cudaMemcpyDeviceToHost,
-                             c->stream));
-  ASOHF_CUDA(cudaMemcpyAsync(indcs + 2 * (size_t)h0, m.d.indcs + 2 * (size_t)h0, 8 * (size_t)(n - h0),
-                             cudaMemcpyDeviceToHost, c->stream));
   if (nslots)
     ASOHF_CUDA(cudaMemcpyAsync(nbound, d_nbound, 4 * (size_t)nslots, cudaMemcpyDeviceToHost, c->stream));
   ASOHF_CUDA(cudaStreamSynchronize(c->stream));
-  for (int i = 0; i < low2 - low1 + 1; i++) slot_of[i] = -1;
+  auto live = [&](int i) { return i < h0 ? m.h.realclus[i] : realclus[i - h0]; };
+  std::vector<int32_t> slot_of((size_t)nw, -1);
   for (int s = 0; s < nslots; s++) slot_of[work[s] - (low1 - 1)] = s;
   int64_t j = 0;
-  for (int i = 1; i < low1; i++)
-    if (realclus[i - 1] != 0 && indcs[(i - 1) * 2 + 1] > j) j = indcs[(i - 1) * 2 + 1];
-  for (int i = low1; i <= low2; i++) {
-    if (realclus[i - 1] == 0) {
-      indcs[(i - 1) * 2] = -1;
-      indcs[(i - 1) * 2 + 1] = -1;
+  for (int i = 0; i < low1 - 1; i++)
+    if (live(i) != 0 && indcs[i * 2 + 1] > j) j = indcs[i * 2 + 1];
+  for (int i = low1 - 1; i < low2; i++) {
+    const int s = slot_of[i - (low1 - 1)];
+    if (live(i) == 0) {
+      indcs[i * 2] = -1;
+      indcs[i * 2 + 1] = -1;
+      if (s >= 0) ids_off[s] = 0;
       continue;
     }
-    int s = slot_of[i - low1];
-    indcs[(i - 1) * 2] = (int32_t)(j + 1);
+    indcs[i * 2] = (int32_t)(j + 1);
     if (s >= 0) {
       ids_off[s] = j;
       j += nbound[s];
     }
-    indcs[(i - 1) * 2 + 1] = (int32_t)j;
+    indcs[i * 2 + 1] = (int32_t)j;
   }
-  for (int s = 0; s < nslots; s++)
-    if (realclus[work[s]] == 0) ids_off[s] = 0;
-  ASOHF_CUDA(cudaMemcpyAsync(m.d.indcs + 2 * (size_t)(low1 - 1), indcs + 2 * (size_t)(low1 - 1),
-                             8 * (size_t)(low2 - low1 + 1), cudaMemcpyHostToDevice, c->stream));
+  if (!m.host) {
+    ASOHF_CUDA(cudaMemcpyAsync(m.d.indcs + 2 * (size_t)(low1 - 1), indcs + 2 * (size_t)(low1 - 1), 8 * (size_t)nw,
+                               cudaMemcpyHostToDevice, c->stream));
+    ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  }
   if (nslots)
     ASOHF_CUDA(cudaMemcpyAsync(d_ids_off, ids_off, 8 * (size_t)nslots, cudaMemcpyHostToDevice, c->stream));
-  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
   *total_out = j;
   return ASOHF_OK;
 }
@@ -1994,13 +2044,17 @@ int assign_id_offsets(asohf_ctx* c, CatMirror& m, int low1, int low2, const int3
 int make_work(asohf_ctx* c, CatMirror& m, int low1, int low2, std::vector<int32_t>& h_work, int* nslots,
               std::vector<int32_t>* h_dm = nullptr) {
   int nh = low2 - low1 + 1;
-  std::vector<int32_t> rc_v((size_t)nh);
-  int32_t* rc = rc_v.data();
-  std::vector<int32_t> dm_v((size_t)nh);
-  int32_t* dm = dm_v.data();
-  ASOHF_CUDA(cudaMemcpyAsync(rc, m.d.realclus + low1 - 1, 4 * (size_t)nh, cudaMemcpyDeviceToHost, c->stream));
-  ASOHF_CUDA(cudaMemcpyAsync(dm, m.d.dmpclus + low1 - 1, 4 * (size_t)nh, cudaMemcpyDeviceToHost, c->stream));
-  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  std::vector<int32_t> rc_v, dm_v;
+  const int32_t *rc = m.h.realclus + low1 - 1, *dm = m.h.dmpclus + low1 - 1;
+  if (!m.host) {
+    rc_v.resize((size_t)nh);
+    dm_v.resize((size_t)nh);
+    ASOHF_CUDA(cudaMemcpyAsync(rc_v.data(), rc, 4 * (size_t)nh, cudaMemcpyDeviceToHost, c->stream));
+    ASOHF_CUDA(cudaMemcpyAsync(dm_v.data(), dm, 4 * (size_t)nh, cudaMemcpyDeviceToHost, c->stream));
+    ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+    rc = rc_v.data();
+    dm = dm_v.data();
+  }
   h_work.assign(nh > 0 ? nh : 1, 0);
   int32_t* w = h_work.data();
   int k = 0;
@@ -2149,6 +2203,7 @@ extern "C" int asohf_halofind_particles(asohf_ctx* c, const asohf_consts* k, con
   int nh = lowh2 - lowh1 + 1;
   size_t need = cat_bytes(lowh2) + (size_t)nh * (96 + 40) + 65536;
   ASOHF_CHECK(arena_reserve(c, need));
+  ASOHF_CHECK(hst_reserve(c, (on_device ? 4 * (size_t)lowh2 : cat_stage_bytes(nh)) + 96 * (size_t)nh + 65536));
   CatMirror m;
   ASOHF_CHECK(cat_mirror_in(c, cat, lowh2, on_device, &m, lowh1 - 1));
   std::vector<int32_t> hw_v, hdm_v;
@@ -2189,17 +2244,18 @@ extern "C" int asohf_halofind_particles(asohf_ctx* c, const asohf_consts* k, con
         !d_ids_off) {
       return ASOHF_ERR_CAPACITY;
     }
-    ASOHF_CUDA(cudaMemcpyAsync(d_work, hw, 4 * (size_t)ns, cudaMemcpyHostToDevice, c->stream));
+    // the host arrays the copies below read and write, page-locked
+    int32_t* hws = (int32_t*)hst_alloc(c, 4 * (size_t)ns);
+    int32_t* hk = (int32_t*)hst_alloc(c, 4 * (size_t)ns);
+    int32_t* hst = (int32_t*)hst_alloc(c, 4 * (size_t)ns);
+    int64_t* hoff = (int64_t*)hst_alloc(c, 8 * (size_t)(ns + 1));
+    if (!hws || !hk || !hst || !hoff) return ASOHF_ERR_CAPACITY;
+    memcpy(hws, hw, 4 * (size_t)ns);
+    ASOHF_CUDA(cudaMemcpyAsync(d_work, hws, 4 * (size_t)ns, cudaMemcpyHostToDevice, c->stream));
     // growth, tiered first by DMPCLUS (the members counted when the candidate
     // was pruned); haloes that outgrow their group size resume in a larger one
     Tiers tg, tm;
     GrowCaps caps{c->tier2_k, 4 * c->tier2_k, CB > 1 ? c->cluster_min : (int64_t)LLONG_MAX};
-    std::vector<int32_t> hk_v((size_t)ns);
-    int32_t* hk = hk_v.data();
-    std::vector<int32_t> hst_v((size_t)ns);
-    int32_t* hst = hst_v.data();
-    std::vector<int64_t> hoff_v((size_t)(ns + 1));
-    int64_t* hoff = hoff_v.data();
     std::vector<int32_t> hesc_v((size_t)ns);
     int32_t* hesc = hesc_v.data();
     std::vector<int32_t> kesc_v((size_t)ns);
@@ -2294,7 +2350,6 @@ extern "C" int asohf_halofind_particles(asohf_ctx* c, const asohf_consts* k, con
     }
     sg.keys = k1;
     sg.vals = v1;
-    ASOHF_CUDA(cudaStreamSynchronize(c->stream));
     htime_end(c, "host:halo_gather_sort", ht);
     ht = htime_now();
     {
@@ -2368,7 +2423,6 @@ extern "C" int asohf_halofind_particles(asohf_ctx* c, const asohf_consts* k, con
   htime_end(c, "host:halo_ids", ht);
   ht = htime_now();
   ASOHF_CHECK(cat_mirror_out(c, &m));
-  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
   htime_end(c, "host:halo_mirror_out", ht);
   return rc;
 }
@@ -2898,13 +2952,19 @@ k_sub_main_g(const int32_t* __restrict__ slots, Store S, HConst H, asohf_catalog
 static int make_sub_work(asohf_ctx* c, CatMirror& m, int low1, int low2, std::vector<int32_t>& h_work,
                          int* nslots) {
   int nh = low2 - low1 + 1;
-  std::vector<int32_t> rc_v((size_t)nh);
-  int32_t* rc = rc_v.data();
-  std::vector<float> rs_v((size_t)nh);
-  float* rs = rs_v.data();
-  ASOHF_CUDA(cudaMemcpyAsync(rc, m.d.realclus + low1 - 1, 4 * (size_t)nh, cudaMemcpyDeviceToHost, c->stream));
-  ASOHF_CUDA(cudaMemcpyAsync(rs, m.d.rsub + low1 - 1, 4 * (size_t)nh, cudaMemcpyDeviceToHost, c->stream));
-  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  std::vector<int32_t> rc_v;
+  std::vector<float> rs_v;
+  const int32_t* rc = m.h.realclus + low1 - 1;
+  const float* rs = m.h.rsub + low1 - 1;
+  if (!m.host) {
+    rc_v.resize((size_t)nh);
+    rs_v.resize((size_t)nh);
+    ASOHF_CUDA(cudaMemcpyAsync(rc_v.data(), rc, 4 * (size_t)nh, cudaMemcpyDeviceToHost, c->stream));
+    ASOHF_CUDA(cudaMemcpyAsync(rs_v.data(), rs, 4 * (size_t)nh, cudaMemcpyDeviceToHost, c->stream));
+    ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+    rc = rc_v.data();
+    rs = rs_v.data();
+  }
   h_work.assign(nh > 0 ? nh : 1, 0);
   int32_t* w = h_work.data();
   int k = 0;
@@ -2924,37 +2984,26 @@ static int make_sub_work(asohf_ctx* c, CatMirror& m, int low1, int low2, std::ve
   return ASOHF_OK;
 }
 
-// gather + segmented sort of the members of `na` spheres (active list act);
-// keys/vals sorted in segments at offsets off (device).
-// Counts, tiers (by count) of the spheres, gathers into segments and sorts
-// them; d_tslots and d_fill hold na entries.
+// Counts the members of `na` spheres (d_act = 0 .. na-1), gathers them into
+// segments at offsets off and sorts these; h_off and hk (page-locked) and
+// d_fill hold na + 1, na and na entries.
 static int gather_sorted(asohf_ctx* c, const Store& S, const ColIdx& ci, int na, const int32_t* d_act,
                          const float* cx, const float* cy, const float* cz, const float* r,
-                         int32_t* d_konta, int64_t* d_off, int64_t* h_off, unsigned long long** keys,
-                         int32_t** vals, int64_t* total, bool with_work, Tiers* tiers, int32_t* d_tslots,
-                         int32_t* d_fill) {
+                         int32_t* d_konta, int64_t* d_off, int64_t* h_off, int32_t* hk, unsigned long long** keys,
+                         int32_t** vals, int64_t* total, Tiers* tiers, int32_t* d_fill) {
   {
     int kt_ = ktime_begin(c, "sub_sphere_count");
     k_sphere_count<<<na, HB, 0, c->stream>>>(ci, d_act, cx, cy, cz, r, d_konta);
     ktime_end(c, kt_);
   }
   c->launches++;
-  std::vector<int32_t> hk_v((size_t)na);
-  int32_t* hk = hk_v.data();
   ASOHF_CUDA(cudaMemcpyAsync(hk, d_konta, 4 * (size_t)na, cudaMemcpyDeviceToHost, c->stream));
   ASOHF_CUDA(cudaStreamSynchronize(c->stream));
   h_off[0] = 0;
   for (int s = 0; s < na; s++) h_off[s + 1] = h_off[s] + hk[s];
   // few subhaloes per call, each in a dense region: 256-thread CTAs (tier 2)
-  // keep more of the GPU busy than the small tiers
-  for (int s = 0; s < na; s++) hk[s] = 0;
-  int64_t keep_t1 = c->tier1_k, keep_t2 = c->tier2_k;
-  c->tier1_k = 0;
-  c->tier2_k = 0;
-  int rt = split_tiers(c, hk, na, d_tslots, tiers);
-  c->tier1_k = keep_t1;
-  c->tier2_k = keep_t2;
-  ASOHF_CHECK(rt);
+  // keep more of the GPU busy than the small tiers.  d_act is 0 .. na-1.
+  *tiers = Tiers{{0, 0, na, 0}, {nullptr, nullptr, const_cast<int32_t*>(d_act), nullptr}};
   int64_t T = h_off[na];
   ASOHF_CUDA(cudaMemcpyAsync(d_off, h_off, 8 * (size_t)(na + 1), cudaMemcpyHostToDevice, c->stream));
   int bits = 1;
@@ -2962,8 +3011,7 @@ static int gather_sorted(asohf_ctx* c, const Store& S, const ColIdx& ci, int na,
   size_t tb = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, tb, (unsigned long long*)nullptr, (unsigned long long*)nullptr,
                                   (int32_t*)nullptr, (int32_t*)nullptr, (int)(T > 0 ? T : 1), 0, 32 + bits);
-  size_t work = with_work ? ((size_t)T + na) * (2 * (8 + 16 + 16) + 8 + 1) + 16384 : 0;
-  ASOHF_CHECK(seg_reserve(c, (size_t)T * 24 + tb + work + 16384));
+  ASOHF_CHECK(seg_reserve(c, (size_t)T * 24 + tb + 16384));
   unsigned long long* k0 = (unsigned long long*)seg_alloc(c, 8 * (size_t)T + 8);
   unsigned long long* k1 = (unsigned long long*)seg_alloc(c, 8 * (size_t)T + 8);
   int32_t* v0 = (int32_t*)seg_alloc(c, 4 * (size_t)T + 4);
@@ -3007,9 +3055,15 @@ __global__ void k_iota32(int32_t* __restrict__ a, int n) {
   if (i < n) a[i] = i;
 }
 
-__global__ void k_gather_f(const int32_t* __restrict__ act, int na, const float* __restrict__ src, float* __restrict__ dst) {
+__global__ void k_gather_spheres(const int32_t* __restrict__ act, int na, SubPrep p, float* __restrict__ cx,
+                                 float* __restrict__ cy, float* __restrict__ cz, float* __restrict__ r) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < na) dst[i] = src[act[i]];
+  if (i >= na) return;
+  const int s = act[i];
+  cx[i] = p.cx[s];
+  cy[i] = p.cy[s];
+  cz[i] = p.cz[s];
+  r[i] = p.r[s];
 }
 
 // Copies segment b of (keys, vals) at off[b] (cnt[b] entries) to dst[b] of
@@ -3069,6 +3123,7 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
   int nh = lowh2 - lowh1 + 1;
   size_t need = cat_bytes(cat->nclus) + (size_t)nh * (192 + 40) + 65536;
   ASOHF_CHECK(arena_reserve(c, need));
+  ASOHF_CHECK(hst_reserve(c, (on_device ? 4 * (size_t)cat->nclus : cat_bytes(cat->nclus)) + 128 * (size_t)nh + 65536));
   CatMirror m;
   ASOHF_CHECK(cat_mirror_in(c, cat, cat->nclus, on_device, &m, lowh1 - 1, true));
   std::vector<int32_t> hw_v;
@@ -3104,19 +3159,22 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
     int32_t* d_nbound = (int32_t*)arena_alloc(c, 4 * (size_t)ns);
     int32_t* d_nscan = (int32_t*)arena_alloc(c, 4 * (size_t)ns);
     int64_t* d_ids_off = (int64_t*)arena_alloc(c, 8 * (size_t)ns);
-    std::vector<int64_t> h_off_v((size_t)(ns + 1));
-    int64_t* h_off = h_off_v.data();
-    std::vector<int32_t> h_act_v((size_t)ns);
-    int32_t* h_act = h_act_v.data();
-    std::vector<int32_t> h_done_v((size_t)ns);
-    int32_t* h_done = h_done_v.data();
-    std::vector<int32_t> h_st_v((size_t)ns);
-    int32_t* h_st = h_st_v.data();
+    // the host arrays the copies below read and write, page-locked
+    int32_t* hws = (int32_t*)hst_alloc(c, 4 * (size_t)ns);
+    int64_t* h_off = (int64_t*)hst_alloc(c, 8 * (size_t)(ns + 1));
+    int64_t* h_dst = (int64_t*)hst_alloc(c, 8 * (size_t)ns);
+    int64_t* fin_off = (int64_t*)hst_alloc(c, 8 * (size_t)ns);
+    int32_t* h_act = (int32_t*)hst_alloc(c, 4 * (size_t)ns);
+    int32_t* h_done = (int32_t*)hst_alloc(c, 4 * (size_t)ns);
+    int32_t* h_st = (int32_t*)hst_alloc(c, 4 * (size_t)ns);
+    int32_t* h_kon = (int32_t*)hst_alloc(c, 4 * (size_t)ns);
+    if (!hws || !h_off || !h_dst || !fin_off || !h_act || !h_done || !h_st || !h_kon) return ASOHF_ERR_CAPACITY;
+    memcpy(hws, hw, 4 * (size_t)ns);
     if (!d_work || !pr.cx || !pr.status || !d_act || !d_konta || !d_off || !t_r || !jo.done || !jo.rclus ||
         !f_jjac || !f_masadm || !f_rclus || !f_rlast || !d_nbound || !d_nscan || !d_ids_off) {
       return ASOHF_ERR_CAPACITY;
     }
-    ASOHF_CUDA(cudaMemcpyAsync(d_work, hw, 4 * (size_t)ns, cudaMemcpyHostToDevice, c->stream));
+    ASOHF_CUDA(cudaMemcpyAsync(d_work, hws, 4 * (size_t)ns, cudaMemcpyHostToDevice, c->stream));
     {
       int kt_ = ktime_begin(c, "sub_prep");
       k_sub_prep<<<ns, HB, 0, c->stream>>>(S, ci, H, m.d, d_work, pr);
@@ -3134,30 +3192,27 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
     ht = htime_now();
     // Jacobi radius, growing the unresolved ones
     int32_t* d_pos = (int32_t*)arena_alloc(c, 4 * (size_t)ns);
-    int32_t* d_tsl = (int32_t*)arena_alloc(c, 4 * (size_t)ns);
     int32_t* d_fill = (int32_t*)arena_alloc(c, 4 * (size_t)ns);
-    if (!d_pos || !d_tsl || !d_fill) rc = ASOHF_ERR_CAPACITY;
+    if (!d_pos || !d_fill) rc = ASOHF_ERR_CAPACITY;
     else k_iota32<<<(ns + 255) / 256, 256, 0, c->stream>>>(d_pos, ns);
-    std::vector<int64_t> fin_off((size_t)ns, 0), fin_cnt((size_t)ns, 0), h_dst((size_t)ns, -1);
+    std::vector<int64_t> fin_cnt((size_t)ns, 0);
+    for (int s = 0; s < ns; s++) { fin_off[s] = 0; h_dst[s] = -1; }
     int64_t fin_total = 0;
     for (int iter = 0; na > 0 && rc == ASOHF_OK; iter++) {
       if (iter > 200) { rc = ASOHF_ERR_TIMEOUT; break; }
       ASOHF_CUDA(cudaMemcpyAsync(d_act, h_act, 4 * (size_t)na, cudaMemcpyHostToDevice, c->stream));
       {
         int kt_ = ktime_begin(c, "sub_jacobi_prep");
-        k_gather_f<<<(na + 255) / 256, 256, 0, c->stream>>>(d_act, na, pr.cx, t_cx);
-        k_gather_f<<<(na + 255) / 256, 256, 0, c->stream>>>(d_act, na, pr.cy, t_cy);
-        k_gather_f<<<(na + 255) / 256, 256, 0, c->stream>>>(d_act, na, pr.cz, t_cz);
-        k_gather_f<<<(na + 255) / 256, 256, 0, c->stream>>>(d_act, na, pr.r, t_r);
+        k_gather_spheres<<<(na + 255) / 256, 256, 0, c->stream>>>(d_act, na, pr, t_cx, t_cy, t_cz, t_r);
         ktime_end(c, kt_);
       }
-      c->launches += 4;
+      c->launches++;
       unsigned long long* keys;
       int32_t* vals;
       int64_t T;
       Tiers tj;
-      ASOHF_CHECK(gather_sorted(c, S, ci, na, d_pos, t_cx, t_cy, t_cz, t_r, d_konta, d_off, h_off, &keys, &vals,
-                                &T, false, &tj, d_tsl, d_fill));
+      ASOHF_CHECK(gather_sorted(c, S, ci, na, d_pos, t_cx, t_cy, t_cz, t_r, d_konta, d_off, h_off, h_kon, &keys,
+                                &vals, &T, &tj, d_fill));
       {
         int kt_ = ktime_begin(c, "sub_jacobi");
         LAUNCH_TIERS_CTA(k_sub_jacobi, tj, S, H, d_act, d_konta, d_off, keys, vals, pr.mhost, pr.disthost, pr.r,
@@ -3189,7 +3244,7 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
       }
       if (fin_total > fin0) {
         ASOHF_CHECK(sfin_reserve(c, fin_total, fin0));
-        ASOHF_CUDA(cudaMemcpyAsync(d_ids_off, h_dst.data(), 8 * (size_t)na, cudaMemcpyHostToDevice, c->stream));
+        ASOHF_CUDA(cudaMemcpyAsync(d_ids_off, h_dst, 8 * (size_t)na, cudaMemcpyHostToDevice, c->stream));
         int kt_ = ktime_begin(c, "sub_keep_segments");
         k_copy_segments<<<na, 256, 0, c->stream>>>(keys, vals, d_off, d_konta, d_ids_off, c->sfin_k, c->sfin_v);
         ktime_end(c, kt_);
@@ -3215,10 +3270,11 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
       int32_t* vals = (int32_t*)seg_alloc(c, 4 * (size_t)T + 4);
       int64_t* d_src = (int64_t*)seg_alloc(c, 8 * (size_t)ns);
       if (!keys || !vals || !d_src) return ASOHF_ERR_CAPACITY;
-      for (int s = 0; s < ns; s++) { h_dst[s] = h_off[s]; h_st[s] = (int32_t)fin_cnt[s]; }
-      ASOHF_CUDA(cudaMemcpyAsync(d_src, fin_off.data(), 8 * (size_t)ns, cudaMemcpyHostToDevice, c->stream));
-      ASOHF_CUDA(cudaMemcpyAsync(d_ids_off, h_dst.data(), 8 * (size_t)ns, cudaMemcpyHostToDevice, c->stream));
-      ASOHF_CUDA(cudaMemcpyAsync(d_konta, h_st, 4 * (size_t)ns, cudaMemcpyHostToDevice, c->stream));
+      ASOHF_CUDA(cudaStreamSynchronize(c->stream));  // the last round's copy of h_dst
+      for (int s = 0; s < ns; s++) { h_dst[s] = h_off[s]; h_kon[s] = (int32_t)fin_cnt[s]; }
+      ASOHF_CUDA(cudaMemcpyAsync(d_src, fin_off, 8 * (size_t)ns, cudaMemcpyHostToDevice, c->stream));
+      ASOHF_CUDA(cudaMemcpyAsync(d_ids_off, h_dst, 8 * (size_t)ns, cudaMemcpyHostToDevice, c->stream));
+      ASOHF_CUDA(cudaMemcpyAsync(d_konta, h_kon, 4 * (size_t)ns, cudaMemcpyHostToDevice, c->stream));
       ASOHF_CUDA(cudaMemcpyAsync(d_off, h_off, 8 * (size_t)(ns + 1), cudaMemcpyHostToDevice, c->stream));
       if (T > 0) {
         int kt_ = ktime_begin(c, "sub_final_segments");
@@ -3227,7 +3283,6 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
         c->launches++;
       }
       ASOHF_CUDA(cudaGetLastError());
-      ASOHF_CUDA(cudaStreamSynchronize(c->stream));
       htime_end(c, "host:sub_final_gather", ht);
       ht = htime_now();
       // staged lists of the kept members, tiers by that count
@@ -3304,8 +3359,7 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
   }
   htime_end(c, "host:sub_ids", ht);
   ht = htime_now();
-  ASOHF_CHECK(cat_mirror_out(c, &m));
-  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  ASOHF_CHECK(cat_mirror_out(c, &m, true));
   htime_end(c, "host:sub_mirror_out", ht);
   return rc;
 }
