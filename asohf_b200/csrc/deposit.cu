@@ -2236,51 +2236,117 @@ __global__ void k_mesh_border(int32_t* __restrict__ cnt, int nx, int bor) {
   }
 }
 
-// One CTA per patch of the level: counts in shared memory (NAMRX^3 ints),
-// candidates from the bins covering the patch widened by two fine cells
-// (a superset of the particles the FLOOR test keeps, for cells wider than
-// the float spacing of the coordinates).
-__global__ void __launch_bounds__(PD_BLOCK)
-k_mesh_patch_counts(const int32_t* __restrict__ pn, const float* __restrict__ pr, int np, Bins B,
-                    const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ z,
-                    int irpa, float dxpa, int refine_thr, int boramr, EspEnds E, int32_t* __restrict__ out) {
-  extern __shared__ int32_t s_cnt[];
-  const int ip = blockIdx.x;
-  const int n1 = pn[ip], n2 = pn[np + ip], n3 = pn[2 * np + ip];
-  for (int q = threadIdx.x; q < NA * NA * NA; q += blockDim.x) s_cnt[q] = 0;
-  __syncthreads();
+// Patches of the level in units of MZ planes: int32 counts in shared memory,
+// candidates from the binned store (x, y, z, weight) over the bins covering the
+// unit widened by two fine cells (a superset of the particles the FLOOR test
+// keeps, for cells wider than the float spacing of the coordinates), in slices
+// as in the deposits; the slices of a unit add to the output, cleared before.
+// Bound by the candidate scan: 2500 patches of 4.1M particles take 0.38 ms (1.29
+// ms with one CTA a patch reading positions through the bin's index).
+#define MZ 8
+#define MSLAB (NA / MZ)
+
+struct MeshPatches {
+  const int32_t* n;  // PATCHNX, Y, Z
+  const float* r;    // PATCHRX, Y, Z
+  int np, boramr;
+  float dxpa;
+};
+
+__device__ __forceinline__ void mesh_unit_geo(const MeshPatches& M, const Bins& B, int u, UnitGeo& g) {
+  g.ip = u / MSLAB;
+  g.slab = u % MSLAB;
+  g.n1 = M.n[g.ip]; g.n2 = M.n[M.np + g.ip]; g.n3 = M.n[2 * M.np + g.ip];
+  g.zlo = g.slab * MZ;  // 0-based planes zlo .. zhi
+  g.zhi = min(g.zlo + MZ, g.n3) - 1;
+  g.dxpa = M.dxpa;
   // XL = PATCHRX - DXPA (grids.f:358-360)
-  const float xl = __fsub_rn(pr[ip], dxpa), yl = __fsub_rn(pr[np + ip], dxpa), zl = __fsub_rn(pr[2 * np + ip], dxpa);
-  const float pad = 2.0f * dxpa;
-  const int bx0 = bin_of(xl - pad, B.xl, B.bsz, B.nb), bx1 = bin_of(xl + (float)(n1 + 2) * dxpa, B.xl, B.bsz, B.nb);
-  const int by0 = bin_of(yl - pad, B.xl, B.bsz, B.nb), by1 = bin_of(yl + (float)(n2 + 2) * dxpa, B.xl, B.bsz, B.nb);
-  const int bz0 = bin_of(zl - pad, B.xl, B.bsz, B.nb), bz1 = bin_of(zl + (float)(n3 + 2) * dxpa, B.xl, B.bsz, B.nb);
-  for (int bz = bz0; bz <= bz1; bz++)
-    for (int by = by0; by <= by1; by++) {
-      const int lo = B.start[(bz * B.nb + by) * B.nb + bx0], hi = B.start[(bz * B.nb + by) * B.nb + bx1 + 1];
-      for (int t = lo + threadIdx.x; t < hi; t += blockDim.x) {
-        const int p = B.idx[t];
-        // IX = FLOOR((RXPA-XL)/DXPA)+1 kept when 1 <= IX <= N1
-        const float vx = __fdiv_rn(__fsub_rn(x[p], xl), dxpa);
-        if (!(vx >= 0.0f && vx < (float)n1)) continue;
-        const float vy = __fdiv_rn(__fsub_rn(y[p], yl), dxpa);
-        if (!(vy >= 0.0f && vy < (float)n2)) continue;
-        const float vz = __fdiv_rn(__fsub_rn(z[p], zl), dxpa);
-        if (!(vz >= 0.0f && vz < (float)n3)) continue;
-        const int w = plev_of(p, E) <= irpa ? 1 : refine_thr;
-        atomicAdd(&s_cnt[((int)vz * NA + (int)vy) * NA + (int)vx], w);
-      }
-    }
-  __syncthreads();
-  int32_t* o = out + (size_t)ip * NA * NA * NA;
-  for (int q = threadIdx.x; q < NA * NA * NA; q += blockDim.x) {
-    const int ix = q % NA + 1, jy = (q / NA) % NA + 1, kz = q / (NA * NA) + 1;
-    int v = s_cnt[q];
-    if (ix > n1 || jy > n2 || kz > n3 || ix <= boramr || ix >= n1 - boramr + 1 || jy <= boramr ||
-        jy >= n2 - boramr + 1 || kz <= boramr || kz >= n3 - boramr + 1)
-      v = 0;
-    o[q] = v;
+  g.xlfix = __fsub_rn(M.r[g.ip], M.dxpa);
+  g.ylfix = __fsub_rn(M.r[M.np + g.ip], M.dxpa);
+  g.zlfix = __fsub_rn(M.r[2 * M.np + g.ip], M.dxpa);
+  const float pad = 2.0f * M.dxpa;
+  g.bx0 = bin_of(g.xlfix - pad, B.xl, B.bsz, B.nb);
+  g.bx1 = bin_of(g.xlfix + (float)(g.n1 + 2) * M.dxpa, B.xl, B.bsz, B.nb);
+  g.by0 = bin_of(g.ylfix - pad, B.xl, B.bsz, B.nb);
+  g.by1 = bin_of(g.ylfix + (float)(g.n2 + 2) * M.dxpa, B.xl, B.bsz, B.nb);
+  g.bz0 = bin_of(g.zlfix + (float)(g.zlo - 2) * M.dxpa, B.xl, B.bsz, B.nb);
+  g.bz1 = bin_of(g.zlfix + (float)(g.zhi + 3) * M.dxpa, B.xl, B.bsz, B.nb);
+  g.nby = g.by1 - g.by0 + 1;
+  g.rows = g.zlo > g.zhi ? 0 : g.nby * (g.bz1 - g.bz0 + 1);
+}
+
+__global__ void k_mesh_unit_counts(MeshPatches M, Bins B, int nunits, uint32_t* __restrict__ key,
+                                   int32_t* __restrict__ unit) {
+  const int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (u >= nunits) return;
+  UnitGeo g;
+  mesh_unit_geo(M, B, u, g);
+  unit_count(B, g, u, lane, key, unit);
+}
+
+// The store in bin order with each particle's weight on the level.
+__global__ void k_mesh_stage(const int32_t* __restrict__ idx, int64_t n, const float* __restrict__ x,
+                             const float* __restrict__ y, const float* __restrict__ z,
+                             const float4* __restrict__ rows, int irpa, int refine_thr, EspEnds E,
+                             float4* __restrict__ P) {
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
+    const int p = idx[t];
+    float4 v = rows ? rows[2 * (int64_t)p] : make_float4(x[p], y[p], z[p], 0.f);
+    v.w = __int_as_float(plev_of(p, E) <= irpa ? 1 : refine_thr);
+    P[t] = v;
   }
+}
+
+__global__ void __launch_bounds__(256)
+k_mesh_patch_counts(MeshPatches M, Bins B, const float4* __restrict__ P, PatchWork W, int32_t* __restrict__ out) {
+  __shared__ int32_t s_cnt[MZ * NA * NA];
+  __shared__ int s_lo[PROWS], s_pre[PROWS + 1];
+  const int2 it = W.items[blockIdx.x];
+  UnitGeo g;
+  mesh_unit_geo(M, B, it.x, g);
+  for (int q = threadIdx.x; q < MZ * NA * NA; q += blockDim.x) s_cnt[q] = 0;
+  const int64_t v0 = (int64_t)it.y * PSLICE, v1 = v0 + PSLICE;
+  int64_t vbase = 0;
+  for (int r0 = 0; r0 < g.rows; r0 += PROWS) {
+    const int nr = min(PROWS, g.rows - r0);
+    __syncthreads();
+    stage_rows(B, g, r0, nr, s_lo, s_pre);
+    __syncthreads();
+    const int tot = s_pre[nr];
+    const int a = (int)(max(v0, vbase) - vbase), b = (int)(min(v1, vbase + tot) - vbase);
+    for (int v = a + threadIdx.x; v < b; v += blockDim.x) {
+      const int row = find_row(s_pre, nr, v);
+      const float4 p = P[s_lo[row] + (v - s_pre[row])];
+      // IX = FLOOR((RXPA-XL)/DXPA)+1 kept when 1 <= IX <= N1
+      const float vz = __fdiv_rn(__fsub_rn(p.z, g.zlfix), g.dxpa);
+      if (!(vz >= 0.0f && vz < (float)g.n3) || (int)vz < g.zlo || (int)vz > g.zhi) continue;
+      const float vx = __fdiv_rn(__fsub_rn(p.x, g.xlfix), g.dxpa);
+      if (!(vx >= 0.0f && vx < (float)g.n1)) continue;
+      const float vy = __fdiv_rn(__fsub_rn(p.y, g.ylfix), g.dxpa);
+      if (!(vy >= 0.0f && vy < (float)g.n2)) continue;
+      atomicAdd(&s_cnt[(((int)vz - g.zlo) * NA + (int)vy) * NA + (int)vx], __float_as_int(p.w));
+    }
+    vbase += tot;
+  }
+  __syncthreads();
+  const bool shared = W.scratch_of[it.x] >= 0;
+  const int bor = M.boramr;
+  int32_t* o = out + ((size_t)g.ip * NA + g.zlo) * NA * NA;
+  for (int q = threadIdx.x; q < MZ * NA * NA; q += blockDim.x) {
+    const int ix = q % NA + 1, jy = (q / NA) % NA + 1, kz = g.zlo + q / (NA * NA) + 1;
+    int v = s_cnt[q];
+    if (ix > g.n1 || jy > g.n2 || kz > g.n3 || ix <= bor || ix >= g.n1 - bor + 1 || jy <= bor ||
+        jy >= g.n2 - bor + 1 || kz <= bor || kz >= g.n3 - bor + 1)
+      v = 0;
+    if (!shared) o[q] = v;
+    else if (v) atomicAdd(&o[q], v);
+  }
+}
+
+// Clears the output of the units that several slices share.
+__global__ void k_mesh_clear(const int32_t* __restrict__ multi, int32_t* __restrict__ out) {
+  int32_t* o = out + (size_t)multi[blockIdx.x] * MZ * NA * NA;
+  for (int q = threadIdx.x; q < MZ * NA * NA; q += blockDim.x) o[q] = 0;
 }
 
 static int esp_ends(const int32_t* npart_esp, EspEnds* E) {
@@ -2338,7 +2404,9 @@ extern "C" int asohf_mesh_patch_counts(asohf_ctx* c, int nx, float lado0, float 
   arena_reset(c);
   const int64_t n = c->p.n;
   const size_t outb = 4 * (size_t)npatch * NA * NA * NA;
-  ASOHF_CHECK(arena_reserve(c, (on_device ? 0 : outb) + 24 * (size_t)npatch + bins_bytes(n, lado0, dx, 2) + 8192));
+  const int nunits = MSLAB * npatch;
+  ASOHF_CHECK(arena_reserve(c, (on_device ? 0 : outb) + (24 + 4 * MSLAB) * (size_t)npatch + 16 * (size_t)n +
+                                   unit_list_bytes(nunits) + bins_bytes(n, lado0, dx, 2) + 16384));
   int32_t* pn = (int32_t*)arena_alloc(c, 12 * (size_t)npatch);
   float* pr = (float*)arena_alloc(c, 12 * (size_t)npatch);
   int32_t* d = on_device ? cr01 : (int32_t*)arena_alloc(c, outb);
@@ -2352,12 +2420,25 @@ extern "C" int asohf_mesh_patch_counts(asohf_ctx* c, int nx, float lado0, float 
   Bins B;
   ASOHF_CHECK(build_bins(c, lado0, dx, 2, &B));
   const float dxpa = ldexpf(dx, -irpa);  // DX/(2.0**IRPA), exact
-  const size_t smem = sizeof(int32_t) * NA * NA * NA;
-  ASOHF_CUDA(cudaFuncSetAttribute(k_mesh_patch_counts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  float4* bp = (float4*)arena_alloc(c, 16 * (size_t)n + 16);
+  if (!bp) return ASOHF_ERR_CAPACITY;
+  const MeshPatches M{pn, pr, npatch, boramr, dxpa};
+  UnitList U;
+  ASOHF_CHECK(unit_list_begin(c, nunits, &U));
   int kt_ = ktime_begin(c, "mesh_patch_counts");
-  k_mesh_patch_counts<<<npatch, PD_BLOCK, smem, c->stream>>>(pn, pr, npatch, B, c->p.x, c->p.y, c->p.z, irpa, dxpa,
-                                                             refine_thr, boramr, E, d);
-  c->launches++;
+  if (n > 0)
+    k_mesh_stage<<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(
+        B.idx, n, c->p.x, c->p.y, c->p.z, c->rows_cur >= 0 ? c->rows[c->rows_cur] : nullptr, irpa, refine_thr, E, bp);
+  k_mesh_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, nunits, U.key, U.unit);
+  ASOHF_CHECK(unit_list_size(c, &U));
+  ASOHF_CHECK(seg_reserve(c, unit_work_bytes(U, 0)));
+  PatchWork W;
+  int32_t* multi;
+  ASOHF_CHECK(unit_list_fill(c, U, 0, [&](size_t b) { return seg_alloc(c, b); },
+                             [&](size_t b) { return arena_alloc(c, b); }, &W, &multi));
+  if (U.nmulti) k_mesh_clear<<<U.nmulti, 256, 0, c->stream>>>(multi, d);
+  k_mesh_patch_counts<<<(unsigned)U.nitems, 256, 0, c->stream>>>(M, B, bp, W, d);
+  c->launches += 2 + (n > 0) + (U.nmulti > 0);
   ktime_end(c, kt_);
   ASOHF_CUDA(cudaGetLastError());
   if (!on_device) ASOHF_CUDA(cudaMemcpyAsync(cr01, d, outb, cudaMemcpyDeviceToHost, c->stream));
@@ -2394,19 +2475,22 @@ __device__ __forceinline__ bool veins_meet(const int32_t* g1, const int32_t* pn,
   return ok;
 }
 
-// Neighbours of each patch, in index order: counts (fill == nullptr) or the list.
+// Neighbours of each patch, in index order: counts (fill == nullptr) or the
+// list.  One warp per patch, 32 partners a step.
 __global__ void k_veins_neighbours(const int32_t* __restrict__ g1, const int32_t* __restrict__ pn, int np,
                                    int32_t* __restrict__ cnt, const int32_t* __restrict__ off,
                                    int32_t* __restrict__ fill) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (i >= np) return;
   int k = 0;
-  for (int j = 0; j < np; j++) {
-    if (j == i || !veins_meet(g1, pn, np, i, j)) continue;
-    if (fill) fill[off[i] + k] = j;
-    k++;
+  for (int j0 = 0; j0 < np; j0 += 32) {
+    const int j = j0 + lane;
+    const bool in = j < np && j != i && veins_meet(g1, pn, np, i, j);
+    const unsigned msk = __ballot_sync(0xffffffffu, in);
+    if (fill && in) fill[off[i] + k + __popc(msk & ((1u << lane) - 1u))] = j;
+    k += __popc(msk);
   }
-  if (!fill) cnt[i] = k;
+  if (!fill && lane == 0) cnt[i] = k;
 }
 
 // The overlap corners of one axis (the four cases of grids.f:1965-2026).
@@ -2438,7 +2522,10 @@ __device__ __forceinline__ void veins_axis_d(float r1, float r2, float rr1, floa
   }
 }
 
-// One CTA per row of the wave: patch I against each neighbour J.
+// A wave's rows, patch I against each neighbour J: one CTA per (J, row).  The
+// pairs of a wave do not depend on one another: a row reads its own patch's
+// marks, which no row of its wave writes.  (One CTA per row walked its
+// neighbours in turn: 2500 level-1 patches of a 160^3 box 1.17 ms, so 0.22.)
 __global__ void __launch_bounds__(256) k_veins_rows(const int32_t* __restrict__ rows, const int32_t* __restrict__ off,
                                                     const int32_t* __restrict__ nb, const int32_t* __restrict__ pn,
                                                     const float* __restrict__ pr, int np, float dxpa,
@@ -2453,7 +2540,7 @@ __global__ void __launch_bounds__(256) k_veins_rows(const int32_t* __restrict__ 
     r1[a] = __fsub_rn(pr[a * np + i], __fmul_rn(0.5f, dxpa));
     r2[a] = __fadd_rn(r1[a], __fmul_rn((float)(n[a] - 1), dxpa));
   }
-  for (int k = off[i]; k < off[i + 1]; k++) {
+  for (int k = off[i] + blockIdx.y; k < off[i + 1]; k += gridDim.y) {
     const int j = nb[k];
     int c1[3], c2[3], cc1[3], cc2[3], e[3];
     for (int a = 0; a < 3; a++) {
@@ -2533,7 +2620,7 @@ extern "C" int asohf_veinsgrid_reduced(asohf_ctx* c, int ir, float dx, float rad
   const float fix = radx1 - dx * 0.5f + 0.5f * dxpa;        // RXFIX
   int kt_ = ktime_begin(c, "veinsgrid_reduced");
   k_veins_box<<<(3 * np + 255) / 256, 256, 0, c->stream>>>(pn, pr, np, dxpa, fix, g1);
-  k_veins_neighbours<<<(np + 127) / 128, 128, 0, c->stream>>>(g1, pn, np, cnt, nullptr, nullptr);
+  k_veins_neighbours<<<(np + 7) / 8, 256, 0, c->stream>>>(g1, pn, np, cnt, nullptr, nullptr);
   ASOHF_CUDA(cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, off, np + 1, c->stream));
   c->launches += 3;
   std::vector<int32_t> hoff(np + 1);
@@ -2552,7 +2639,7 @@ extern "C" int asohf_veinsgrid_reduced(asohf_ctx* c, int ir, float dx, float rad
     ASOHF_CHECK(seg_reserve(c, 4 * (size_t)ne + 256));
     nb = (int32_t*)seg_alloc(c, 4 * (size_t)ne);
     if (!nb) return ASOHF_ERR_CAPACITY;
-    k_veins_neighbours<<<(np + 127) / 128, 128, 0, c->stream>>>(g1, pn, np, nullptr, off, nb);
+    k_veins_neighbours<<<(np + 7) / 8, 256, 0, c->stream>>>(g1, pn, np, nullptr, off, nb);
     c->launches++;
   }
   std::vector<int32_t> hnb(ne > 0 ? ne : 1);
@@ -2569,7 +2656,11 @@ extern "C" int asohf_veinsgrid_reduced(asohf_ctx* c, int ir, float dx, float rad
     nwave = std::max(nwave, w + 1);
   }
   std::vector<int32_t> wstart(nwave + 1, 0), horder(np);
-  for (int i = 0; i < np; i++) wstart[wave[i] + 1]++;
+  std::vector<int> wmax(nwave, 0);  // most neighbours of a row of the wave
+  for (int i = 0; i < np; i++) {
+    wstart[wave[i] + 1]++;
+    wmax[wave[i]] = std::max(wmax[wave[i]], hoff[i + 1] - hoff[i]);
+  }
   for (int w = 0; w < nwave; w++) wstart[w + 1] += wstart[w];
   {
     std::vector<int32_t> fillp(wstart.begin(), wstart.end() - 1);
@@ -2579,7 +2670,8 @@ extern "C" int asohf_veinsgrid_reduced(asohf_ctx* c, int ir, float dx, float rad
   for (int w = 0; w < nwave; w++) {
     const int nr = wstart[w + 1] - wstart[w];
     if (nr <= 0) continue;
-    k_veins_rows<<<nr, 256, 0, c->stream>>>(rows + wstart[w], off, nb, pn, pr, np, dxpa, solap, dcr, dct);
+    const dim3 grid((unsigned)nr, (unsigned)std::max(1, std::min(wmax[w], 65535)));
+    k_veins_rows<<<grid, 256, 0, c->stream>>>(rows + wstart[w], off, nb, pn, pr, np, dxpa, solap, dcr, dct);
     c->launches++;
   }
   ktime_end(c, kt_);
