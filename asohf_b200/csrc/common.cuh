@@ -138,6 +138,11 @@ struct asohf_ctx {
   bool dens_pending = false;
   struct Pool { char* base = nullptr; size_t size = 0, used = 0; };
   Pool dpool[2];
+  // COMPUTE_KERNELS' tables for interpolation degree 1 and 2, levels 0 ..
+  // kern_nl (the same for every call): on the host, and on the device
+  float* h_kern[2] = {nullptr, nullptr};
+  float* d_kern[2] = {nullptr, nullptr};
+  int kern_nl[2] = {-1, -1};
   // device copies kept between calls: MOMENTO's sin^2 table for s2_nx, and
   // the last RADX(0:NX+1) the layer was given (h_radx: its host copy)
   float* d_s2 = nullptr;

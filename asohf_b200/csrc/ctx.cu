@@ -289,6 +289,10 @@ extern "C" int asohf_destroy(asohf_ctx* c) {
   free_particles(c->stage);
   cudaFree(c->rows[0]);
   cudaFree(c->rows[1]);
+  for (int d = 0; d < 2; d++) {
+    cudaFree(c->d_kern[d]);
+    free(c->h_kern[d]);
+  }
   cudaFree(c->d_s2);
   cudaFree(c->d_tw);
   cudaFree(c->d_radx);
