@@ -223,18 +223,40 @@ static HConst hconst(const asohf_consts* k, const asohf_mesh* mesh) {
 }
 
 // ---------------------------------------------------------------- prune
-// COUNT_PARTICLES_HALO (haloes_particles.f:147-182) for haloes low1..low2.
-__global__ void __launch_bounds__(HB) k_prune(ColIdx ci, asohf_catalogue cat, int low1, float facrad,
-                                             int min_num_part) {
+// CTAs that share the count of one sphere (blockIdx.y): those past one for
+// every QPART_COLS columns of its box have nothing to add and leave at once.
+// One CTA a halo left the largest ones running alone: the 1102 + 1121 + 429
+// haloes of 128^3 particles took 1.20 ms in four calls, and 0.43 so.
+#define QPARTS 8
+#define QPART_COLS 6
+
+// The columns the box of r around a centre meets, and this CTA's part of the
+// warps that share them; false when the part is empty.
+__device__ __forceinline__ bool query_part(const ColIdx& ci, float cy, float cz, float r, int* w0, int* nw) {
+  const float rr = r * 1.0001f + 1e-6f;
+  const int ny = col_index(cy + rr, ci.xl, ci.cdx, ci.ncol) - col_index(cy - rr, ci.xl, ci.cdx, ci.ncol) + 1;
+  const int nz = col_index(cz + rr, ci.xl, ci.cdx, ci.ncol) - col_index(cz - rr, ci.xl, ci.cdx, ci.ncol) + 1;
+  const int parts = min((int)gridDim.y, max(1, ny * nz / QPART_COLS));
+  const int per = blockDim.x >> 5;
+  *w0 = blockIdx.y * per + (threadIdx.x >> 5);
+  *nw = parts * per;
+  return (int)blockIdx.y < parts;
+}
+
+// COUNT_PARTICLES_HALO (haloes_particles.f:147-182) for haloes low1..low2,
+// added to DMPCLUS (cleared before).
+__global__ void __launch_bounds__(HB) k_prune(ColIdx ci, asohf_catalogue cat, int low1, float facrad) {
   __shared__ long long lred[32];
   int i0 = low1 - 1 + blockIdx.x;
   float cx = cat.clusrx[i0], cy = cat.clusry[i0], cz = cat.clusrz[i0];
   float r = __fmul_rn(facrad, cat.radio[i0]);
   float r2 = __fmul_rn(r, r);
+  int w0, nw;
+  if (!query_part(ci, cy, cz, r, &w0, &nw)) return;
   int64_t lo, hi;
   slab_range(ci, cx, r, &lo, &hi);
   long long cnt = 0;
-  query_box(ci, cx, cy, cz, r, [&](const float4& e) {
+  query_box_w(ci, cx, cy, cz, r, w0, nw, [&](const float4& e) {
     int p = ppos(e);
     if (p < lo || p >= hi) return;
     float bx = __fsub_rn(e.x, cx);
@@ -249,10 +271,7 @@ __global__ void __launch_bounds__(HB) k_prune(ColIdx ci, asohf_catalogue cat, in
     if (__fadd_rn(__fadd_rn(bx, by), bz) < r2) cnt++;
   });
   cnt = block_sum_ll(cnt, lred);
-  if (threadIdx.x == 0) {
-    if (cnt < min_num_part) cat.realclus[i0] = 0;
-    cat.dmpclus[i0] = (int32_t)cnt;
-  }
+  if (threadIdx.x == 0 && cnt) atomicAdd(&cat.dmpclus[i0], (int32_t)cnt);
 }
 
 __global__ void k_prune_nocount(asohf_catalogue cat, int low1, int low2, int min_num_part) {
@@ -274,14 +293,14 @@ extern "C" int asohf_prune_poor_haloes(asohf_ctx* c, const asohf_consts* k, asoh
   CatMirror m;
   ASOHF_CHECK(cat_mirror_in(c, cat, low2, on_device, &m, low1 - 1, false, true));
   int nh = low2 - low1 + 1;
-  if (do_need_to_count == 1)
-    {
-      int kt_ = ktime_begin(c, "prune");
-      k_prune<<<nh, HB, 0, c->stream>>>(col_idx(c, k), m.d, low1, facrad, k->min_num_part);
-      ktime_end(c, kt_);
-    }
-  else
-    k_prune_nocount<<<(nh + 255) / 256, 256, 0, c->stream>>>(m.d, low1, low2, k->min_num_part);
+  if (do_need_to_count == 1) {
+    int kt_ = ktime_begin(c, "prune");
+    ASOHF_CUDA(cudaMemsetAsync(m.d.dmpclus + low1 - 1, 0, 4 * (size_t)nh, c->stream));
+    k_prune<<<dim3(nh, QPARTS), HB, 0, c->stream>>>(col_idx(c, k), m.d, low1, facrad);
+    ktime_end(c, kt_);
+    c->launches++;
+  }
+  k_prune_nocount<<<(nh + 255) / 256, 256, 0, c->stream>>>(m.d, low1, low2, k->min_num_part);
   c->launches++;
   ASOHF_CUDA(cudaGetLastError());
   ASOHF_CHECK(cat_mirror_out(c, &m));
@@ -2501,24 +2520,26 @@ k_sub_prep(Store S, ColIdx ci, HConst H, asohf_catalogue cat, const int32_t* __r
   o.status[slot] = 0;
 }
 
-// Members of the sphere r around the centre (count only).
+// Members of the sphere r around the centre (count only), added to konta
+// (cleared before); blockIdx.y as in k_prune.
 __global__ void __launch_bounds__(HB)
 k_sphere_count(ColIdx ci, const int32_t* __restrict__ act, const float* __restrict__ hcx,
                const float* __restrict__ hcy, const float* __restrict__ hcz, const float* __restrict__ r,
                int32_t* __restrict__ konta) {
   __shared__ long long lred[32];
-  __shared__ QBuf qb;
   int s = act[blockIdx.x];
   float cx = hcx[s], cy = hcy[s], cz = hcz[s], rr = r[s];
+  int w0, nw;
+  if (!query_part(ci, cy, cz, rr, &w0, &nw)) return;
   int64_t lo, hi;
   slab_range(ci, cx, rr, &lo, &hi);
   long long c = 0;
-  gquery_box(Grp<1>(), ci, cx, cy, cz, rr, qb, [&](const float4& e) {
+  query_box_w(ci, cx, cy, cz, rr, w0, nw, [&](const float4& e) {
     int p = ppos(e);
     if (p >= lo && p < hi && dist3(e.x, e.y, e.z, cx, cy, cz) < rr) c++;
   });
   c = block_sum_ll(c, lred);
-  if (threadIdx.x == 0) konta[blockIdx.x] = (int32_t)c;
+  if (threadIdx.x == 0 && c) atomicAdd(&konta[blockIdx.x], (int32_t)c);
 }
 
 __device__ __forceinline__ double eq_jacobi_dev(double basx, double basy) {
@@ -2993,7 +3014,8 @@ static int gather_sorted(asohf_ctx* c, const Store& S, const ColIdx& ci, int na,
                          int32_t** vals, int64_t* total, Tiers* tiers, int32_t* d_fill) {
   {
     int kt_ = ktime_begin(c, "sub_sphere_count");
-    k_sphere_count<<<na, HB, 0, c->stream>>>(ci, d_act, cx, cy, cz, r, d_konta);
+    ASOHF_CUDA(cudaMemsetAsync(d_konta, 0, 4 * (size_t)na, c->stream));
+    k_sphere_count<<<dim3(na, QPARTS), HB, 0, c->stream>>>(ci, d_act, cx, cy, cz, r, d_konta);
     ktime_end(c, kt_);
   }
   c->launches++;
@@ -3022,8 +3044,14 @@ static int gather_sorted(asohf_ctx* c, const Store& S, const ColIdx& ci, int na,
     // the per-sphere arrays are indexed by position in the active list
     ASOHF_CUDA(cudaMemsetAsync(d_fill, 0, 4 * (size_t)na, c->stream));
     {
+      // few spheres, some of them in the cores of clusters: a thread-block
+      // cluster each (a CTA each left the largest alone: with the counts split
+      // as above, the Jacobi rounds of 313 subhaloes 6.7 against 4.5 ms)
       int kt_ = ktime_begin(c, "sub_gather");
-      LAUNCH_TIERS_CTA(k_halo_gather, *tiers, S, ci, d_konta, d_off, cx, cy, cz, r, d_fill, k0, v0);
+      const int C = big_cluster(c) >= 8 ? 8 : 1;
+      ASOHF_CUDA(LAUNCH_TIER(k_halo_gather, C, na, c->stream, d_act, S, ci, d_konta, d_off, cx, cy, cz, r, d_fill,
+                             k0, v0));
+      c->launches++;
       ktime_end(c, kt_);
     }
     int kt_ = ktime_begin(c, "sub_radix_sort");
