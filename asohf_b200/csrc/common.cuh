@@ -56,8 +56,9 @@ struct asohf_ctx {
   int num_sms = 148;
   // size tiers of the per-halo launches (members): >= cluster_min a CTA
   // cluster, >= tier2_k 256 threads, >= tier1_k 128 threads, else 32
-  int64_t cluster_min = 32768;
-  int64_t cluster_share = 32768;  // entries per CTA that set the halo kernel's cluster width
+  int64_t cluster_min = 0;    // 0: by the call's members (cluster_rule)
+  int64_t cluster_share = 0;  // entries per CTA that set the halo kernel's cluster width; 0 likewise
+  int64_t eff_min = 32768, eff_share = 32768;  // what the running call uses
   int64_t tier2_k = 2048, tier1_k = 256;
   // seed of COMPUTE_EPOT's sampling estimator (asohf_set_epot_seed)
   uint32_t epot_seed = 1;

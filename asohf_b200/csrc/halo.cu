@@ -310,12 +310,13 @@ extern "C" int asohf_prune_poor_haloes(asohf_ctx* c, const asohf_consts* k, asoh
 
 // ---------------------------------------------------------------- launch helpers
 // Size tiers of the per-halo launches, by member count: at least
-// ctx->cluster_min -> a thread-block cluster; at least ctx->tier2_k -> one
+// ctx->eff_min -> a thread-block cluster; at least ctx->tier2_k -> one
 // CTA of 256 threads; at least ctx->tier1_k -> 128 threads; the rest -> 32
 // threads.  The small CTAs keep many small haloes resident per SM, whose
 // passes are short and bound by latency.  The tiers run concurrently on four
 // streams.
 #define BIG_K 32768
+#define SMALL_K 2048
 #define TIER2_K 2048
 #define TIER1_K 256
 static const int kTierThreads[3] = {32, 128, 256};
@@ -357,6 +358,19 @@ static int join_all(asohf_ctx* c) {
   return ASOHF_OK;
 }
 
+// Cluster threshold and share of a call over `members` particles, where they
+// were not set: a halo of more than 1/256 of them outlasts the others on one
+// CTA (148 SMs hold a few hundred), so small calls take clusters from 2048
+// members on and large ones from 32768.  Whole catalogues with 2048 or 8192,
+// and with 32768, for both: 64^3 6.0 and 6.9 ms, 128^3 14.5 and 16.4, 256^3 (16384)
+// 38.9 and 39.9.
+static void cluster_rule(asohf_ctx* c, int64_t members) {
+  int64_t k = members / 256;
+  k = k < SMALL_K ? SMALL_K : (k > BIG_K ? BIG_K : k);
+  c->eff_min = c->cluster_min > 0 ? c->cluster_min : (k < c->tier2_k ? c->tier2_k : k);
+  c->eff_share = c->cluster_share > 0 ? c->cluster_share : k;
+}
+
 struct Tiers {
   int n[4];           // slots per tier (0: 32 threads, 1: 128, 2: 256, 3: cluster)
   int32_t* slots[4];  // device slot lists
@@ -375,7 +389,7 @@ static int split_tiers(asohf_ctx* c, const int32_t* hcount, int n, int32_t* dbuf
   }
   int cnt[4] = {0, 0, 0, 0};
   auto tier = [&](int32_t k) {
-    return k >= c->cluster_min ? 3 : (k >= c->tier2_k ? 2 : (k >= c->tier1_k ? 1 : 0));
+    return k >= c->eff_min ? 3 : (k >= c->tier2_k ? 2 : (k >= c->tier1_k ? 1 : 0));
   };
   for (int i = 0; i < n; i++) cnt[tier(hcount[i])]++;
   int off[4];
@@ -396,10 +410,10 @@ static int split_tiers(asohf_ctx* c, const int32_t* hcount, int n, int32_t* dbuf
 
 // Reorders the cluster tier's slot list (tier 3, at the front of its
 // device buffer) into runs for clusters of cb (at most 16), 8 and 4 CTAs by
-// member count: a CTA's share stays near ctx->cluster_share entries.
+// member count: a CTA's share stays near ctx->eff_share entries.
 static int split_cluster_tier(asohf_ctx* c, const int32_t* hcount, int n, int cb, Tiers* T, int nsub[3],
                               int32_t* sub[3]) {
-  const int64_t sh = c->cluster_share;
+  const int64_t sh = c->eff_share;
   auto pick = [&](int32_t k) {
     if (cb < 8) return 0;                      // no clusters: one CTA each
     if (cb < 16) return k > 4 * sh ? 0 : 2;  // 8 CTAs at most
@@ -414,10 +428,10 @@ static int split_cluster_tier(asohf_ctx* c, const int32_t* hcount, int n, int cb
   }
   int cnt[3] = {0, 0, 0};
   for (int i = 0; i < n; i++)
-    if (hcount[i] >= c->cluster_min) cnt[pick(hcount[i])]++;
+    if (hcount[i] >= c->eff_min) cnt[pick(hcount[i])]++;
   int fill[3] = {0, cnt[0], cnt[0] + cnt[1]};
   for (int i = 0; i < n; i++)
-    if (hcount[i] >= c->cluster_min) h[fill[pick(hcount[i])]++] = i;
+    if (hcount[i] >= c->eff_min) h[fill[pick(hcount[i])]++] = i;
   if (T->n[3]) ASOHF_CUDA(cudaMemcpyAsync(T->slots[3], h, 4 * (size_t)T->n[3], cudaMemcpyHostToDevice, c->stream));
   if (!staged) ASOHF_CUDA(cudaStreamSynchronize(c->stream));
   for (int q = 0; q < 3; q++) {
@@ -2191,13 +2205,13 @@ extern "C" int asohf_set_epot_seed(asohf_ctx* c, uint32_t seed) {
 
 extern "C" int asohf_set_cluster_threshold(asohf_ctx* c, int64_t min_members) {
   if (!c || min_members < 0) return ASOHF_ERR_INVALID;
-  c->cluster_min = min_members == 0 ? BIG_K : min_members;
+  c->cluster_min = min_members;
   return ASOHF_OK;
 }
 
 extern "C" int asohf_set_cluster_share(asohf_ctx* c, int64_t members_per_cta) {
   if (!c || members_per_cta < 0) return ASOHF_ERR_INVALID;
-  c->cluster_share = members_per_cta == 0 ? 32768 : members_per_cta;
+  c->cluster_share = members_per_cta;
   return ASOHF_OK;
 }
 
@@ -2273,8 +2287,11 @@ extern "C" int asohf_halofind_particles(asohf_ctx* c, const asohf_consts* k, con
     ASOHF_CUDA(cudaMemcpyAsync(d_work, hws, 4 * (size_t)ns, cudaMemcpyHostToDevice, c->stream));
     // growth, tiered first by DMPCLUS (the members counted when the candidate
     // was pruned); haloes that outgrow their group size resume in a larger one
+    int64_t members = 0;
+    for (int s = 0; s < ns; s++) members += hdm[s] > 0 ? hdm[s] : 0;
+    cluster_rule(c, members);
     Tiers tg, tm;
-    GrowCaps caps{c->tier2_k, 4 * c->tier2_k, CB > 1 ? c->cluster_min : (int64_t)LLONG_MAX};
+    GrowCaps caps{c->tier2_k, 4 * c->tier2_k, CB > 1 ? c->eff_min : (int64_t)LLONG_MAX};
     std::vector<int32_t> hesc_v((size_t)ns);
     int32_t* hesc = hesc_v.data();
     std::vector<int32_t> kesc_v((size_t)ns);
@@ -3164,6 +3181,7 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
   ColIdx ci = col_idx(c, k);
   HConst H = hconst(k, mesh);
   H.epot_seed = c->epot_seed;
+  cluster_rule(c, 256 * (int64_t)BIG_K);  // single CTAs only: the largest threshold
   int rc = ASOHF_OK;
   if (ns > 0) {
     int32_t* d_work = (int32_t*)arena_alloc(c, 4 * (size_t)ns);
