@@ -1695,7 +1695,7 @@ k_halo_main(const int32_t* __restrict__ slots, Store S, HConst H, asohf_catalogu
                            __fdiv_rn(__fmul_rn(4.0f, pi), 3.0f));
     float cvir = __fmul_rn(H.contrastec, fdm);
     long long best = LLONG_MAX;
-    gscan_d(g, 0, idx_vir, 0.0, [&](int64_t j) { return (double)cur.dm[j].y; },
+    gscan_unit(g, idx_vir, (double)S.meq, [&](int64_t j) { return (double)cur.dm[j].y; },
               [&](int64_t j, double menc) {
                 if (j + 1 <= jjcore) return;
                 float d = cur.dm[j].x;
@@ -1784,7 +1784,8 @@ k_halo_main(const int32_t* __restrict__ slots, Store S, HConst H, asohf_catalogu
   // passes, which read it instead of scanning again
   long long jt[7];
   for (int q = 0; q < 7; q++) jt[q] = LLONG_MAX;
-  gscan_d(g, 0, k2, 0.0, mn_of,
+  const double unit = S.meq != 0.0f ? (double)__fdiv_rn(S.meq, norma) : 0.0;  // one mass: its share of NORMA
+  gscan_unit(g, k2, unit, mn_of,
             [&](int64_t j, double bas8) {
               pot[j] = bas8;
               int64_t J = j + 1;
@@ -2583,7 +2584,8 @@ k_sub_jacobi(const int32_t* __restrict__ slots, Store S, HConst H, const int32_t
              const float* __restrict__ disthost_a, float* __restrict__ r, JacOut o) {
   static_assert(C == 1, "one CTA per subhalo");
   __shared__ MainShared sh;
-  __shared__ double s_m[4];
+  __shared__ double s_m;
+  __shared__ unsigned long long s_found;
   int b = slots[blockIdx.x], s = act[b];
   int64_t K = konta[b];
   const unsigned long long* kk = keys + off[b];
@@ -2596,61 +2598,92 @@ k_sub_jacobi(const int32_t* __restrict__ slots, Store S, HConst H, const int32_t
   int64_t minj = max((int64_t)10, K / 50);
   double mh3 = (double)__fmul_rn(3.0f, mhost);
   double expo = (double)(1.0f / 3.0f);
-  // estimation: first J > MINJ with r/D - (m/(m+3M))^(1/3) > 0
-  long long jest = LLONG_MAX;
-  tile_prefix_d(0, K, 0.0, [&](int64_t j) { return (double)S.mass(lip[j]); },
-                [&](int64_t j, double mas) {
-                  int64_t J = j + 1;
-                  if (J <= minj) return;
-                  double mu = mas * um;
-                  double eq = (double)__fdiv_rn(dista(J), disthost) - pow(mu / (mu + mh3), expo);
-                  if (eq > 0.0 && J < jest) jest = J;
-                },
-                sh.dred);
-  jest = bmin(jest, sh);
+  // the searched tests, on the mass of the first J members
+  auto estimate = [&](int64_t J, double mas) {  // r/D - (m/(m+3M))^(1/3) > 0
+    const double mu = mas * um, q = (double)__fdiv_rn(dista(J), disthost), x = mu / (mu + mh3);
+    // far below the root the cubes decide (EXPO is 1/3 within 1e-8, so the
+    // power is the root within 1e-6 for any ratio of masses)
+    if (q * q * q < x * (1.0 - 1e-5)) return false;
+    return q - pow(x, expo) > 0.0;
+  };
+  auto residual = [&](int64_t J, double mas) {
+    return eq_jacobi_dev((double)__fdiv_rn(dista(J), disthost), mas * um / (double)mhost);
+  };
+  // the mass of the first J members: with one particle mass m * J, exactly, so
+  // the searches test only the members up to (or down to) their answer; with
+  // several masses each is a scan of all members
+  const double meq = (double)S.meq;
+  auto first_of = [&](int64_t a, int64_t e, auto test) -> long long {  // first J of [a, e]
+    if (meq == 0.0) {
+      long long f = LLONG_MAX;
+      tile_prefix_d(0, K, 0.0, [&](int64_t j) { return (double)S.mass(lip[j]); },
+                    [&](int64_t j, double mas) {
+                      if (j + 1 >= a && j + 1 <= e && j + 1 < f && test(j + 1, mas)) f = j + 1;
+                    },
+                    sh.dred);
+      return bmin(f, sh);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_found = ~0ull;
+    __syncthreads();
+    for (int64_t J = a + threadIdx.x; J <= e; J += blockDim.x) {
+      if (*(volatile unsigned long long*)&s_found < (unsigned long long)J) break;
+      if (test(J, meq * (double)J)) {
+        atomicMin(&s_found, (unsigned long long)J);
+        break;
+      }
+    }
+    __syncthreads();
+    return s_found == ~0ull ? LLONG_MAX : (long long)s_found;
+  };
+  auto last_of = [&](int64_t a, int64_t e, auto test) -> long long {  // last J of [a, e], -1: none
+    if (meq == 0.0) {
+      long long f = -1;
+      tile_prefix_d(0, K, 0.0, [&](int64_t j) { return (double)S.mass(lip[j]); },
+                    [&](int64_t j, double mas) {
+                      if (j + 1 >= a && j + 1 <= e && j + 1 > f && test(j + 1, mas)) f = j + 1;
+                    },
+                    sh.dred);
+      return -bmin(-f, sh);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) s_found = 0ull;
+    __syncthreads();
+    for (int64_t J = e - threadIdx.x; J >= a; J -= blockDim.x) {
+      if (*(volatile unsigned long long*)&s_found > (unsigned long long)J) break;
+      if (test(J, meq * (double)J)) {
+        atomicMax(&s_found, (unsigned long long)J);
+        break;
+      }
+    }
+    __syncthreads();
+    return s_found == 0ull ? -1 : (long long)s_found;
+  };
+  auto mass_of = [&](int64_t J) -> double {  // 0 outside the members
+    if (meq != 0.0) return J >= 1 && J <= K ? meq * (double)J : 0.0;
+    __syncthreads();
+    if (threadIdx.x == 0) s_m = 0.0;
+    __syncthreads();
+    tile_prefix_d(0, K, 0.0, [&](int64_t j) { return (double)S.mass(lip[j]); },
+                  [&](int64_t j, double mas) { if (j + 1 == J) s_m = mas; }, sh.dred);
+    __syncthreads();
+    return s_m;
+  };
+  const long long jest = first_of(minj + 1, K, estimate);
   int64_t jj = jest == LLONG_MAX ? K : jest;
-  // masses at jj and prefix lookups
-  double mjj = 0.0;
-  if (threadIdx.x == 0) s_m[0] = 0.0;
-  __syncthreads();
-  tile_prefix_d(0, K, 0.0, [&](int64_t j) { return (double)S.mass(lip[j]); },
-                [&](int64_t j, double mas) { if (j + 1 == jj) s_m[0] = mas; }, sh.dred);
-  __syncthreads();
-  mjj = s_m[0];
-  double basx = (double)__fdiv_rn(dista(jj), disthost);
-  double basy = mjj * um / (double)mhost;
-  double eq = eq_jacobi_dev(basx, basy);
+  const double mjj = mass_of(jj);
+  double eq = eq_jacobi_dev((double)__fdiv_rn(dista(jj), disthost), mjj * um / (double)mhost);
   int flag = 0, dir = -1;
   long long jfound = LLONG_MAX;
   double masadm = mjj;
   // ABS(EQ_JACOBI_R).LT.0.D01 compares with 0.0D+01 = 0: never true
   if (eq < 0.0) {
     dir = 1;  // forward: first J > jj with EQ > 0
-    long long f = LLONG_MAX;
-    tile_prefix_d(0, K, 0.0, [&](int64_t j) { return (double)S.mass(lip[j]); },
-                  [&](int64_t j, double mas) {
-                    int64_t J = j + 1;
-                    if (J <= jj) return;
-                    double bx = (double)__fdiv_rn(dista(J), disthost);
-                    double e2 = eq_jacobi_dev(bx, mas * um / (double)mhost);
-                    if (e2 > 0.0 && J < f) f = J;
-                  },
-                  sh.dred);
-    f = bmin(f, sh);
+    const long long f = first_of(jj + 1, K, [&](int64_t J, double mas) { return residual(J, mas) > 0.0; });
     if (f != LLONG_MAX) { flag = 1; jfound = f; }
   } else {
     // backward: largest J in [MINJ, jj-1] with EQ(prefix(J)) < 0
-    long long f = -1;
-    tile_prefix_d(0, K, 0.0, [&](int64_t j) { return (double)S.mass(lip[j]); },
-                  [&](int64_t j, double mas) {
-                    int64_t J = j + 1;
-                    if (J < minj || J > jj - 1) return;
-                    double bx = (double)__fdiv_rn(dista(J), disthost);
-                    double e2 = eq_jacobi_dev(bx, mas * um / (double)mhost);
-                    if (e2 < 0.0 && J > f) f = J;
-                  },
-                  sh.dred);
-    f = -bmin(-f, sh);  // max (-1: none)
+    const long long f = last_of(minj, jj - 1, [&](int64_t J, double mas) { return residual(J, mas) < 0.0; });
     if (f > 0) { flag = 1; jfound = f; }
   }
   int64_t jj2 = jj;
@@ -2664,14 +2697,10 @@ k_sub_jacobi(const int32_t* __restrict__ slots, Store S, HConst H, const int32_t
     // MASADM at the final J: prefix(J) (forward and backward searches) or,
     // when the backward loop ran out, prefix(MINJ); a zero-trip backward
     // loop keeps prefix(jj)
-    if (threadIdx.x == 0) s_m[1] = 0.0;
-    __syncthreads();
     int64_t jm = jj2;
     if (dir == -1 && jfound == LLONG_MAX && jj - 1 < minj) jm = jj;
-    tile_prefix_d(0, K, 0.0, [&](int64_t j) { return (double)S.mass(lip[j]); },
-                  [&](int64_t j, double mas) { if (j + 1 == jm) s_m[1] = mas; }, sh.dred);
-    __syncthreads();
-    masadm = (jm >= 1 && jm <= K) ? s_m[1] : (jm > K ? mjj : 0.0);
+    const double mjm = mass_of(jm);
+    masadm = (jm >= 1 && jm <= K) ? mjm : (jm > K ? mjj : 0.0);
   }
   if (threadIdx.x == 0) {
     o.done[b] = flag;
@@ -2853,7 +2882,7 @@ k_sub_main_g(const int32_t* __restrict__ slots, Store S, HConst H, asohf_catalog
       }
       long long f = -1;
       double mf = 0.0;
-      gscan_d(g, 0, k2, 0.0, [&](int64_t j) { return (double)cur.dm[j].y; },
+      gscan_unit(g, k2, (double)S.meq, [&](int64_t j) { return (double)cur.dm[j].y; },
               [&](int64_t j, double pre) {
                 const int64_t J = j + 1;
                 const double mj = m0 - (tot - pre + (double)cur.dm[j].y);  // after subtracting m(J..K2)
@@ -2896,7 +2925,8 @@ k_sub_main_g(const int32_t* __restrict__ slots, Store S, HConst H, asohf_catalog
   long long best_j = LLONG_MAX;
   double best_b = 0.0;
   auto mn_of = [&](int64_t j) { return (double)__fdiv_rn(cur.dm[j].y, norma); };
-  const double btot = gscan_d(g, 0, k2, 0.0, mn_of,
+  const double unit = S.meq != 0.0f ? (double)__fdiv_rn(S.meq, norma) : 0.0;
+  const double btot = gscan_unit(g, k2, unit, mn_of,
                               [&](int64_t j, double bas8) {
                                 const int64_t J = j + 1;
                                 if (J <= jjcore) return;
@@ -2916,7 +2946,7 @@ k_sub_main_g(const int32_t* __restrict__ slots, Store S, HConst H, asohf_catalog
   // BAS8 at the crossings and the momentum sums, in one more pass
   double sv[10];
   for (int q = 0; q < 10; q++) sv[q] = 0.0;
-  gscan_d(g, 0, k2, 0.0, mn_of,
+  gscan_unit(g, k2, unit, mn_of,
           [&](int64_t j, double bas8) {
             for (int q = 0; q < 7; q++)
               if (j + 1 == jt[q]) sv[q] = bas8;

@@ -983,6 +983,28 @@ __device__ __forceinline__ double gscan_d(const Grp<C>& g, int64_t a, int64_t b,
   return carry + tot;
 }
 
+// gscan_d from 0 over [0, b) of terms that are all `unit` when that is not 0:
+// the prefix at j is unit * (j + 1), exactly (unit holds 24 bits, the count
+// fewer than 29), so the entries are consumed without a scan, each by the thread
+// that would have it there.
+template <int C, class V, class U>
+__device__ __forceinline__ double gscan_unit(const Grp<C>& g, int64_t b, double unit, V val, U use, double* wbuf,
+                                             GX& x) {
+  if (unit == 0.0) return gscan_d(g, 0, b, 0.0, val, use, wbuf, x);
+  int64_t wlo = 0, whi = b;
+  bool one = C == 0;
+  if constexpr (C == 1) one = blockDim.x == 32;
+  if (!one) {
+    int64_t lo, hi;
+    g.chunk(0, b, &lo, &hi);
+    warp_run(lo, hi, &wlo, &whi);
+  }
+  for (int64_t j = wlo + (threadIdx.x & 31); j < whi; j += 32) use(j, unit * (double)(j + 1));
+  if (one) __syncthreads();
+  else g.sync();
+  return unit * (double)b;
+}
+
 // Prefix of the recurrence M_j = M_{j-1} + m_j, Q_j = Q_{j-1} + M_j * w_j
 // (a cumulative mass and a sum weighted by it) in one scan.  A run of
 // entries is summarised by (sum m, sum w, its own Q from zero); runs combine
