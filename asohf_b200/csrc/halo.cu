@@ -2484,7 +2484,8 @@ extern "C" int asohf_get_particles_per_halo(asohf_ctx* c, int32_t* out, int64_t 
 // subhaloes whose radius must grow x1.5; a last gather at the final radius;
 // then k_sub_main_g on the staged lists: unbinding, Jacobi trim, SO walk,
 // properties.  The per-subhalo kernels run in the size tiers of the halo
-// path, single CTAs only.
+// path, the largest subhaloes on clusters of 8 CTAs (the Jacobi searches on
+// single CTAs).
 
 struct SubPrep {
   float *cx, *cy, *cz;
@@ -3017,6 +3018,19 @@ k_sub_main_g(const int32_t* __restrict__ slots, Store S, HConst H, asohf_catalog
   }
 }
 
+// Cluster size of the subhalo kernels on this device: 8 CTAs or one.
+static int sub_cluster(asohf_ctx* c) {
+  static int size[64];
+  const int d = c->device;
+  if (d < 0 || d >= 64) return 1;
+  if (size[d] == 0)
+    size[d] = big_cluster(c) >= 8 && max_clusters(k_sub_main_g<8>, 8) > 0 && max_clusters(k_halo_gather<8>, 8) > 0 &&
+                      max_clusters(k_write_ids<8>, 8) > 0
+                  ? 8
+                  : 1;
+  return size[d];
+}
+
 static int make_sub_work(asohf_ctx* c, CatMirror& m, int low1, int low2, std::vector<int32_t>& h_work,
                          int* nslots) {
   int nh = low2 - low1 + 1;
@@ -3095,8 +3109,7 @@ static int gather_sorted(asohf_ctx* c, const Store& S, const ColIdx& ci, int na,
       // cluster each (a CTA each left the largest alone: with the counts split
       // as above, the Jacobi rounds of 313 subhaloes 6.7 against 4.5 ms)
       int kt_ = ktime_begin(c, "sub_gather");
-      const int C = big_cluster(c) >= 8 ? 8 : 1;
-      ASOHF_CUDA(LAUNCH_TIER(k_halo_gather, C, na, c->stream, d_act, S, ci, d_konta, d_off, cx, cy, cz, r, d_fill,
+      ASOHF_CUDA(LAUNCH_TIER(k_halo_gather, sub_cluster(c), na, c->stream, d_act, S, ci, d_konta, d_off, cx, cy, cz, r, d_fill,
                              k0, v0));
       c->launches++;
       ktime_end(c, kt_);
@@ -3211,7 +3224,8 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
   ColIdx ci = col_idx(c, k);
   HConst H = hconst(k, mesh);
   H.epot_seed = c->epot_seed;
-  cluster_rule(c, 256 * (int64_t)BIG_K);  // single CTAs only: the largest threshold
+  cluster_rule(c, 0);  // few subhaloes a call: clusters from the smallest threshold on
+  const int CS = sub_cluster(c);
   int rc = ASOHF_OK;
   if (ns > 0) {
     int32_t* d_work = (int32_t*)arena_alloc(c, 4 * (size_t)ns);
@@ -3398,7 +3412,7 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
       ASOHF_CHECK(split_tiers(c, h_st, ns, d_ts, &ts));
       {
         int kt_ = ktime_begin(c, "sub_main");
-        LAUNCH_TIERS_CTA(k_sub_main_g, ts, S, H, m.d, d_work, in, sg);
+        LAUNCH_TIERS(k_sub_main_g, CS, ts, S, H, m.d, d_work, in, sg);
         ktime_end(c, kt_);
       }
       {
@@ -3420,8 +3434,8 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
         ASOHF_CHECK(ensure_pph(c, total));
         {
           int kt_ = ktime_begin(c, "sub_write_ids");
-          LAUNCH_TIERS_CTA(k_write_ids, ts, d_nscan, d_off, d_ids_off, sg.final_b, sg.a.px, sg.b.px, sg.flag,
-                           c->p.id, c->d_pph);
+          LAUNCH_TIERS(k_write_ids, CS, ts, d_nscan, d_off, d_ids_off, sg.final_b, sg.a.px, sg.b.px, sg.flag,
+                       c->p.id, c->d_pph);
           ktime_end(c, kt_);
         }
         ASOHF_CUDA(cudaGetLastError());
