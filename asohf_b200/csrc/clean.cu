@@ -433,12 +433,14 @@ int clean_in(asohf_ctx* c, const asohf_catalogue* cat, int n, int on_device, Cle
                      speeds ? cat->vz : nullptr, speeds ? cat->masa : nullptr, cat->radio, cat->levhal, cat->realclus};
     return ASOHF_OK;
   }
-  // one block through page-locked staging: up to 8 fields, levels, REALCLUS
+  // up to 8 fields, levels, REALCLUS: one block through page-locked staging, or
+  // a copy each where they are large
   const void* hf[10] = {cat->clusrx, cat->clusry, cat->clusrz, cat->vx, cat->vy, cat->vz, cat->masa, cat->radio,
                         cat->levhal, cat->realclus};
   const size_t row = (4 * (size_t)n + 15) & ~(size_t)15;
-  ASOHF_CHECK(hst_reserve(c, 11 * row + 1024));
-  char* hb = (char*)hst_alloc(c, 10 * row + 16);
+  const bool direct = 4 * (size_t)n >= HST_DIRECT;
+  ASOHF_CHECK(hst_reserve(c, (direct ? 1 : 11) * row + 1024));
+  char* hb = (char*)hst_alloc(c, direct ? 16 : 10 * row + 16);
   char* db = (char*)arena_alloc(c, 10 * row + 16);
   if (!hb || !db) return ASOHF_ERR_CAPACITY;
   char* df[10];
@@ -447,10 +449,11 @@ int clean_in(asohf_ctx* c, const asohf_catalogue* cat, int n, int on_device, Cle
     df[q] = nullptr;
     if (!speeds && q >= 3 && q <= 6) continue;
     df[q] = db + at;
-    memcpy(hb + at, hf[q], 4 * (size_t)n);
+    if (direct) ASOHF_CUDA(cudaMemcpyAsync(df[q], hf[q], 4 * (size_t)n, cudaMemcpyHostToDevice, c->stream));
+    else memcpy(hb + at, hf[q], 4 * (size_t)n);
     at += row;
   }
-  if (n) ASOHF_CUDA(cudaMemcpyAsync(db, hb, at, cudaMemcpyHostToDevice, c->stream));
+  if (n && !direct) ASOHF_CUDA(cudaMemcpyAsync(db, hb, at, cudaMemcpyHostToDevice, c->stream));
   auto f = [&](int q) { return (const float*)df[q]; };
   io->d = CleanCat{f(0), f(1), f(2), f(3), f(4), f(5), f(6), f(7), (const int32_t*)df[8], (int32_t*)df[9]};
   return ASOHF_OK;

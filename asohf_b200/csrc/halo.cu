@@ -12,12 +12,12 @@
 //   k_halo_main   virial index, escape-velocity and sigma-clipping
 //                 unbinding, SO walk, bound-particle properties;
 //   k_write_ids   bound-particle IDs in halo order (PARTICLES_PER_HALO).
-// Each per-halo kernel runs in two tiers: haloes of 32768 members or more
-// (asohf_set_cluster_threshold)
-// are refined by a thread-block cluster (16 CTAs, or 8 where 16 cannot be
-// co-scheduled) that splits every pass over the members, the others by one
-// CTA each on a second stream, so the clusters and the single CTAs share the
-// SMs instead of the largest halo finishing alone.
+// Each per-halo kernel runs in size tiers: the largest haloes of a call
+// (cluster_rule, asohf_set_cluster_threshold) are refined by a thread-block
+// cluster (16 CTAs, or 8 where 16 cannot be co-scheduled) that splits every
+// pass over the members, the others by one CTA each on other streams, so the
+// clusters and the single CTAs share the SMs instead of the largest halo
+// finishing alone.
 // The reference scans a full-(y,z) x-slab per query (haloes_particles.f:
 // 117-143); the column index returns the same member sets from the columns a
 // sphere overlaps.
@@ -33,11 +33,13 @@
 // ---------------------------------------------------------------- catalogue mirror
 // A call reads and writes the entries of its own haloes, [w0, n), and (the
 // subhalo calls) a few fields of earlier entries, their hosts.  With a host
-// catalogue only those ranges cross PCIe, all fields of a call packed in
-// page-locked staging and moved as one block each way; the device pointers are
-// shifted so that the kernels keep the caller's indexing.  (A copy a field, 45
-// each way, took 1.0 ms of a call's 1.4 ms on the host at a few hundred
-// haloes.)  INDCS is host work and stays there.
+// catalogue only those ranges cross PCIe, fields below HST_DIRECT bytes packed
+// in page-locked staging and moved as one block each way; the device pointers
+// are shifted so that the kernels keep the caller's indexing.  (A copy a field,
+// 45 each way, took 1.0 ms of a call's 1.4 ms on the host at a few hundred
+// haloes; with 200000 haloes packing every field took 7.1 ms in and 8.2 out for
+// the haloes and 9.0 in for the subhaloes, this rule 2.1, 3.5 and 0.4.)  INDCS
+// is host work and stays there.
 struct CatMirror {
   asohf_catalogue h;  // caller's
   asohf_catalogue d;  // device
@@ -46,7 +48,7 @@ struct CatMirror {
   bool host;
   bool prune;         // only the fields PRUNE_POOR_HALOES reads and writes move
   char *hblk, *dblk;  // the packed window fields, staged and on the device
-  size_t bytes;
+  size_t bytes;       // of the packed window fields
 };
 
 #define CAT_F1(X) X(masa) X(radio) X(clusrx) X(clusry) X(clusrz) X(clusrxcm) X(clusrycm) X(clusrzcm) \
@@ -84,8 +86,14 @@ static size_t cat_next(size_t* at, size_t rows, int w) {
   return o;
 }
 
-// Staging a call needs for the mirror of n entries.
-static size_t cat_stage_bytes(int n) { return 2 * cat_bytes(n); }
+static bool cat_direct(size_t rows, int w) { return 4 * rows * (size_t)w >= HST_DIRECT; }
+
+// Staging a call needs for the mirror of n entries: its packed fields, fewer
+// than 64 of less than HST_DIRECT bytes.
+static size_t cat_stage_bytes(int n) {
+  const size_t b = cat_bytes(n), most = 64 * HST_DIRECT;
+  return b < most ? b : most;
+}
 
 static int cat_mirror_in(asohf_ctx* c, asohf_catalogue* h, int n, int on_device, CatMirror* m, int w0,
                          bool hosts = false, bool prune = false) {
@@ -99,11 +107,12 @@ static int cat_mirror_in(asohf_ctx* c, asohf_catalogue* h, int n, int on_device,
   m->d = *h;
   if (on_device) return ASOHF_OK;
   const size_t a = (size_t)m->w0, cnt = (size_t)(n - m->w0);
-  // fields of the window first, in one block; the hosts' fields after it
-  size_t total = 0, hat = 0;
-#define SZ(f, w) if (!(hosts && cat_host_field(#f))) cat_next(&total, cnt, w);
+  // packed fields of the window first, in one block, the hosts' after it, then
+  // the fields that are copied by themselves
+  size_t total = 0, hat = 0, big = 0;
+#define SZ(f, w) if (!(hosts && cat_host_field(#f))) cat_next(cat_direct(cnt, w) ? &big : &total, cnt, w);
 #define SZ1(f) SZ(f, 1)
-#define HZ(f, w) cat_next(&hat, (size_t)n, w);
+#define HZ(f, w) cat_next(cat_direct((size_t)n, w) ? &big : &hat, (size_t)n, w);
   if (prune) { CAT_PRUNE_IN(SZ1) }
   else { CAT_F1(SZ1) CAT_I1(SZ1) CAT_FM(SZ) }
   if (hosts) { CAT_HOST(HZ) }
@@ -111,22 +120,29 @@ static int cat_mirror_in(asohf_ctx* c, asohf_catalogue* h, int n, int on_device,
 #undef SZ1
 #undef HZ
   m->hblk = (char*)hst_alloc(c, total + hat + 16);
-  m->dblk = (char*)arena_alloc(c, total + hat + 16);
+  m->dblk = (char*)arena_alloc(c, total + hat + big + 16);
   if (!m->hblk || !m->dblk) return ASOHF_ERR_CAPACITY;
   m->bytes = total;
-  size_t at = 0;
+  size_t at = 0, bat = total + hat;
+  auto put = [&](const void* src, size_t rows, int w) -> char* {
+    const bool direct = cat_direct(rows, w);
+    const size_t o = cat_next(direct ? &bat : &at, rows, w), b = 4 * rows * (size_t)w;
+    if (!direct) memcpy(m->hblk + o, src, b);
+    else if (cudaMemcpyAsync(m->dblk + o, src, b, cudaMemcpyHostToDevice, c->stream) != cudaSuccess) return nullptr;
+    return m->dblk + o;
+  };
 #define F(f, w)                                                                      \
   if (!(hosts && cat_host_field(#f))) {                                              \
-    const size_t o = cat_next(&at, cnt, w);                                          \
-    memcpy(m->hblk + o, h->f + a * (w), 4 * cnt * (w));                              \
-    m->d.f = (decltype(m->d.f))((uintptr_t)(m->dblk + o) - 4 * a * (w));             \
+    const char* p = put(h->f + a * (w), cnt, w);                                     \
+    if (!p) return ASOHF_ERR_CUDA;                                                   \
+    m->d.f = (decltype(m->d.f))((uintptr_t)p - 4 * a * (w));                         \
   }
 #define F1(f) F(f, 1)
 #define HF(f, w)                                                                     \
   {                                                                                  \
-    const size_t o = cat_next(&at, (size_t)n, w);                                    \
-    memcpy(m->hblk + o, h->f, 4 * (size_t)n * (w));                                  \
-    m->d.f = (decltype(m->d.f))(m->dblk + o);                                        \
+    char* p = put(h->f, (size_t)n, w);                                               \
+    if (!p) return ASOHF_ERR_CUDA;                                                   \
+    m->d.f = (decltype(m->d.f))p;                                                    \
   }
   if (prune) { CAT_PRUNE_IN(F1) }
   else { CAT_F1(F1) CAT_I1(F1) CAT_FM(F) }
@@ -146,6 +162,21 @@ static int cat_mirror_out(asohf_ctx* c, CatMirror* m, bool hosts = false) {
     return ASOHF_OK;
   }
   const size_t a = (size_t)m->w0, cnt = (size_t)(m->n - m->w0);
+  // the fields copied by themselves on the way in
+  auto direct = [&](const char* name, int w) {
+    return cat_direct(hosts && cat_host_field(name) ? (size_t)m->n : cnt, w);
+  };
+#define D(f, w)                                                                                          \
+  if (direct(#f, w))                                                                                     \
+    ASOHF_CUDA(cudaMemcpyAsync(m->h.f + a * (w), m->d.f + a * (w), 4 * cnt * (w), cudaMemcpyDeviceToHost, \
+                               c->stream));
+#define D1(f) D(f, 1)
+  if (m->prune && cat_direct(cnt, 1)) {
+    D1(realclus) D1(dmpclus)
+    ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+    c->hst_busy = false;
+    return ASOHF_OK;
+  }
   if (m->prune) {  // the two last fields of the block
     const size_t f = (4 * cnt + 15) & ~(size_t)15;
     char* b = m->hblk + m->bytes - 2 * f;
@@ -156,20 +187,23 @@ static int cat_mirror_out(asohf_ctx* c, CatMirror* m, bool hosts = false) {
     memcpy(m->h.dmpclus + a, b + f, 4 * cnt);
     return ASOHF_OK;
   }
-  ASOHF_CUDA(cudaMemcpyAsync(m->hblk, m->dblk, m->bytes, cudaMemcpyDeviceToHost, c->stream));
+  if (m->bytes) ASOHF_CUDA(cudaMemcpyAsync(m->hblk, m->dblk, m->bytes, cudaMemcpyDeviceToHost, c->stream));
   if (hosts) {  // the window part of the hosts' fields, into their place in the staging
 #define HF(f, w)                                                                                       \
-  {                                                                                                    \
+  if (!cat_direct((size_t)m->n, w)) {                                                                  \
     const size_t o = (size_t)((char*)m->d.f - m->dblk) + 4 * a * (w);                                  \
     ASOHF_CUDA(cudaMemcpyAsync(m->hblk + o, m->dblk + o, 4 * cnt * (w), cudaMemcpyDeviceToHost, c->stream)); \
   }
     CAT_HOST(HF)
 #undef HF
   }
+  CAT_F1(D1) CAT_I1(D1) CAT_FM(D)
+#undef D
+#undef D1
   ASOHF_CUDA(cudaStreamSynchronize(c->stream));
   c->hst_busy = false;
-#define F(f, w) \
-  memcpy(m->h.f + a * (w), m->hblk + ((char*)(m->d.f + a * (w)) - m->dblk), 4 * cnt * (w));
+#define F(f, w)                            \
+  if (!direct(#f, w)) memcpy(m->h.f + a * (w), m->hblk + ((char*)(m->d.f + a * (w)) - m->dblk), 4 * cnt * (w));
 #define F1(f) F(f, 1)
   CAT_F1(F1) CAT_I1(F1) CAT_FM(F)
 #undef F
@@ -2237,7 +2271,7 @@ extern "C" int asohf_halofind_particles(asohf_ctx* c, const asohf_consts* k, con
   int nh = lowh2 - lowh1 + 1;
   size_t need = cat_bytes(lowh2) + (size_t)nh * (96 + 40) + 65536;
   ASOHF_CHECK(arena_reserve(c, need));
-  ASOHF_CHECK(hst_reserve(c, (on_device ? 4 * (size_t)lowh2 : cat_stage_bytes(nh)) + 96 * (size_t)nh + 65536));
+  ASOHF_CHECK(hst_reserve(c, 4 * (size_t)lowh2 + (on_device ? 0 : cat_stage_bytes(nh)) + 96 * (size_t)nh + 65536));
   CatMirror m;
   ASOHF_CHECK(cat_mirror_in(c, cat, lowh2, on_device, &m, lowh1 - 1));
   std::vector<int32_t> hw_v, hdm_v;
@@ -3211,7 +3245,7 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
   int nh = lowh2 - lowh1 + 1;
   size_t need = cat_bytes(cat->nclus) + (size_t)nh * (192 + 40) + 65536;
   ASOHF_CHECK(arena_reserve(c, need));
-  ASOHF_CHECK(hst_reserve(c, (on_device ? 4 * (size_t)cat->nclus : cat_bytes(cat->nclus)) + 128 * (size_t)nh + 65536));
+  ASOHF_CHECK(hst_reserve(c, 4 * (size_t)cat->nclus + (on_device ? 0 : cat_stage_bytes(cat->nclus)) + 128 * (size_t)nh + 65536));
   CatMirror m;
   ASOHF_CHECK(cat_mirror_in(c, cat, cat->nclus, on_device, &m, lowh1 - 1, true));
   std::vector<int32_t> hw_v;
