@@ -3258,7 +3258,12 @@ extern "C" int asohf_substructure_particles(asohf_ctx* c, const asohf_consts* k,
   ColIdx ci = col_idx(c, k);
   HConst H = hconst(k, mesh);
   H.epot_seed = c->epot_seed;
-  cluster_rule(c, 0);  // few subhaloes a call: clusters from the smallest threshold on
+  // few subhaloes a call: clusters from the smallest threshold on, also where a
+  // larger one was set for the haloes (k_sub_main_g at 512^3 with 65536 set: 6.6
+  // and 3.8 ms a step)
+  cluster_rule(c, 0);
+  const int64_t sub_min = c->tier2_k > SMALL_K ? c->tier2_k : SMALL_K;
+  if (c->eff_min > sub_min) c->eff_min = sub_min;
   const int CS = sub_cluster(c);
   int rc = ASOHF_OK;
   if (ns > 0) {
