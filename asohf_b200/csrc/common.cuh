@@ -194,6 +194,12 @@ void* dpool_alloc(asohf_ctx* c, int which, size_t bytes);
 int density_settle(asohf_ctx* c);
 void* seg_alloc(asohf_ctx* c, size_t bytes);
 
+// A table the context keeps, from host memory: on the context's stream, which
+// the kernels that read it follow (a copy on the legacy stream may end after it
+// returns, and a non-blocking stream does not wait for it), and done before the
+// context can change streams.
+int upload_table(asohf_ctx* c, void* dst, const void* src, size_t bytes);
+
 // Page-locked staging: hst_reserve starts a call's use (contents lost), after
 // waiting for a use that did not clear hst_busy at its end.
 int hst_reserve(asohf_ctx* c, size_t bytes);

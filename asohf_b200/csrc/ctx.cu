@@ -170,6 +170,12 @@ void* seg_alloc(asohf_ctx* c, size_t bytes) {
   return p;
 }
 
+int upload_table(asohf_ctx* c, void* dst, const void* src, size_t bytes) {
+  ASOHF_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream));
+  ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+  return ASOHF_OK;
+}
+
 int hst_reserve(asohf_ctx* c, size_t bytes) {
   c->hst_used = 0;
   if (c->hst_busy) ASOHF_CUDA(cudaStreamSynchronize(c->stream));
@@ -236,7 +242,8 @@ extern "C" int asohf_create(int device, asohf_ctx** out) {
   c->device = device;
   cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device);
   bool ok = arena_reserve(c, 64u << 20) == ASOHF_OK && cudaMalloc(&c->d_work, 64) == cudaSuccess &&
-            cudaMemset(c->d_work, 0, 64) == cudaSuccess &&
+            cudaMemsetAsync(c->d_work, 0, 64, c->stream) == cudaSuccess &&
+            cudaStreamSynchronize(c->stream) == cudaSuccess &&
             cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) == cudaSuccess;
   for (int i = 0; ok && i < asohf_ctx::NSIDE; i++)
     ok = cudaStreamCreateWithFlags(&c->side[i], cudaStreamNonBlocking) == cudaSuccess &&

@@ -69,12 +69,7 @@ static int kernel_tables(asohf_ctx* c, int nl, int deg, const float** hk, float*
   if (l0 <= nl) {
     float* row = c->h_kern[d] + (size_t)l0 * KW;
     for (int ir = l0; ir <= nl; ir++) compute_kernel_level(ir, deg, c->h_kern[d] + (size_t)ir * KW + ASOHF_NMAX_KERNELS);
-    // on the context's stream, which the kernels that read the rows follow (a
-    // copy on the legacy stream may end after it returns, and a non-blocking
-    // stream does not wait for it); done before the context can change streams
-    ASOHF_CUDA(cudaMemcpyAsync(c->d_kern[d] + (size_t)l0 * KW, row, sizeof(float) * KW * (size_t)(nl - l0 + 1),
-                               cudaMemcpyHostToDevice, c->stream));
-    ASOHF_CUDA(cudaStreamSynchronize(c->stream));
+    ASOHF_CHECK(upload_table(c, c->d_kern[d] + (size_t)l0 * KW, row, sizeof(float) * KW * (size_t)(nl - l0 + 1)));
     c->kern_nl[d] = nl;
   }
   *hk = c->h_kern[d];

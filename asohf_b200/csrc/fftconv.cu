@@ -215,8 +215,8 @@ static int twiddles(asohf_ctx* c, int n, const float2** out) {
     h[n / 2] = make_float2(-1.f, 0.f);
     h[3 * n / 4] = make_float2(0.f, 1.f);
     cudaError_t e = cudaMalloc(&c->d_tw, sizeof(float2) * (size_t)n);
-    if (e == cudaSuccess) e = cudaMemcpy(c->d_tw, h.data(), sizeof(float2) * (size_t)n, cudaMemcpyHostToDevice);
     ASOHF_CUDA(e);
+    ASOHF_CHECK(upload_table(c, c->d_tw, h.data(), sizeof(float2) * (size_t)n));
     c->tw_n = n;
   }
   *out = c->d_tw;

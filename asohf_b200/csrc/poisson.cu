@@ -138,8 +138,8 @@ static int green_table(asohf_ctx* c, int nx, const float** out) {
     float* hs2 = hs2_v.data();
     momento_axis(nx, hs2);
     cudaError_t e = cudaMalloc(&c->d_s2, 4 * (size_t)nx);
-    if (e == cudaSuccess) e = cudaMemcpy(c->d_s2, hs2, 4 * (size_t)nx, cudaMemcpyHostToDevice);
     ASOHF_CUDA(e);
+    ASOHF_CHECK(upload_table(c, c->d_s2, hs2, 4 * (size_t)nx));
     c->s2_nx = nx;
   }
   *out = c->d_s2;
@@ -162,7 +162,7 @@ int radx_device(asohf_ctx* c, int nx, const float* radx, const float** out) {
       c->radx_n = n;
     }
     memcpy(c->h_radx, radx, 4 * (size_t)n);
-    ASOHF_CUDA(cudaMemcpy(c->d_radx, radx, 4 * (size_t)n, cudaMemcpyHostToDevice));
+    ASOHF_CHECK(upload_table(c, c->d_radx, c->h_radx, 4 * (size_t)n));
   }
   *out = c->d_radx;
   return ASOHF_OK;

@@ -39,3 +39,32 @@ def test_first_density_on_a_non_blocking_stream(gpu_lib, degree):
     got = _density(s, mesh, degree, torch.cuda.Stream())
     for a, b in zip(got, want):  # float64 sums in any order, rounded once to REAL*4
         assert np.allclose(a, b, rtol=2.0 ** -23, atol=0.0)
+
+
+@pytest.mark.parametrize("nx", [24, 64])
+def test_first_solves_on_a_non_blocking_stream(gpu_lib, nx):
+    g = torch.Generator(device="cuda").manual_seed(nx)
+    L = np.float32(20.0)
+    radx, dx = grid.malla(nx, L)
+    cos = grid.cosmology(0.678, 0.31, 0.0)
+    xyz = [((torch.rand(3000, generator=g, device="cuda") - 0.5) * 0.999 * float(L)) for _ in range(3)]
+    m = torch.ones(3000, device="cuda")
+    rho = torch.randn(nx ** 3, generator=g, device="cuda")
+    got = []
+    for st in (torch.cuda.default_stream(), torch.cuda.Stream()):
+        st.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(st):
+            pot, dep, phi = (torch.empty(nx ** 3, device="cuda") for _ in range(3))
+            for fn in ("poisson", "forward"):  # each the first call of its context
+                a = api.Asohf(0)
+                a.set_stream(st.cuda_stream)
+                if fn == "poisson":
+                    a.poisson_fft(nx, dx, rho, pot)
+                else:
+                    a.tsc_poisson_forward(nx, L, dx, radx, cos["rote"], cos["rete"], *xyz, m, dep, phi, 1)
+                st.synchronize()
+                a.close()
+            got.append([pot, dep, phi])
+    torch.cuda.synchronize()
+    for a, b in zip(*got):  # one plan on both streams; the deposit's float64 sums in any order
+        assert float((a - b).abs().max()) <= 2.0 ** -20 * float(b.abs().max())

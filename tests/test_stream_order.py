@@ -21,7 +21,7 @@ def _code(path):
     return re.sub(r"//[^\n]*", "", s)
 
 
-@pytest.mark.parametrize("name", ["deposit.cu"])
+@pytest.mark.parametrize("name", sorted(os.path.basename(f) for f in glob.glob(os.path.join(CSRC, "*.cu*"))))
 def test_no_copy_on_the_legacy_stream(name):
     files = glob.glob(os.path.join(CSRC, name))
     assert files
