@@ -437,6 +437,8 @@ int clean_in(asohf_ctx* c, const asohf_catalogue* cat, int n, int on_device, Cle
   // a copy each where they are large
   const void* hf[10] = {cat->clusrx, cat->clusry, cat->clusrz, cat->vx, cat->vy, cat->vz, cat->masa, cat->radio,
                         cat->levhal, cat->realclus};
+  for (int q = 0; q < 10; q++)
+    if (n && !hf[q] && (speeds || q < 3 || q > 6)) return ASOHF_ERR_INVALID;
   const size_t row = (4 * (size_t)n + 15) & ~(size_t)15;
   const bool direct = 4 * (size_t)n >= HST_DIRECT;
   ASOHF_CHECK(hst_reserve(c, (direct ? 1 : 11) * row + 1024));

@@ -509,6 +509,8 @@ extern "C" int asohf_halofind_grid_base(asohf_ctx* c, int nx, float dx, const fl
   // the rows into the caller's catalogue (IF (IR.EQ.0) NCLUS=0)
   void* const out[11] = {cat->realclus, cat->levhal, cat->patchclus, cat->clusrx,   cat->clusry,  cat->clusrz,
                          cat->radio,    cat->masa,   cat->clusrxcm,  cat->clusrycm, cat->clusrzcm};
+  for (int q = 0; q < 11; q++)
+    if (nk > 0 && !out[q]) return ASOHF_ERR_INVALID;
   const size_t nb = 4 * (size_t)nk;
   if (nk > 0 && cat_on_device) {
     for (int q = 0; q < 11; q++)

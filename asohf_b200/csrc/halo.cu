@@ -107,6 +107,13 @@ static int cat_mirror_in(asohf_ctx* c, asohf_catalogue* h, int n, int on_device,
   m->d = *h;
   if (on_device) return ASOHF_OK;
   const size_t a = (size_t)m->w0, cnt = (size_t)(n - m->w0);
+  // a missing array is refused here: the packing reads the others on the host
+#define NZ(f, w) if (cnt && !h->f) return ASOHF_ERR_INVALID;
+#define NZ1(f) NZ(f, 1)
+  if (prune) { CAT_PRUNE_IN(NZ1) }
+  else { CAT_F1(NZ1) CAT_I1(NZ1) CAT_FM(NZ) NZ(indcs, 2) }
+#undef NZ
+#undef NZ1
   // packed fields of the window first, in one block, the hosts' after it, then
   // the fields that are copied by themselves
   size_t total = 0, hat = 0, big = 0;
