@@ -13,11 +13,16 @@ others held (coordinate descent), and returns the fastest.  ``apply`` sets a
 choice on a backend; ``save`` and ``load`` keep it per workload signature in
 a JSON file.
 
+``LIBRARY`` is the state of an untouched context: cluster threshold and share
+0, which leaves both to the library's rule for each call's members.
+``tune_plan`` starts from it, checks against it and falls back to it.
+``DEFAULTS`` holds fixed thresholds, those the rule takes for the largest calls.
+
 A setting changes launch shapes only: in every tier the kernels give the
 same integer fields and ID lists, and float fields within float32 rounding
 of the reduction order (1e-5 relative, the parity bar against the oracle).
-``tune_plan`` checks the chosen setting against the default setting's
-catalogue by that bar (``check=True``) and keeps the defaults when it fails.
+``tune_plan`` checks the chosen setting against the untouched library's
+catalogue by that bar (``check=True``) and keeps that state when it fails.
 """
 from __future__ import annotations
 
@@ -27,20 +32,23 @@ import time
 
 import numpy as np
 
+LIBRARY = {"tier1": 256, "tier2": 2048, "cluster_min": 0, "cluster_share": 0}
 DEFAULTS = {"tier1": 256, "tier2": 2048, "cluster_min": 32768, "cluster_share": 32768}
 SPACE = {
     "tier1": [128, 256, 512],
     "tier2": [1024, 2048, 4096],
-    "cluster_min": [16384, 32768, 65536, 131072],
-    "cluster_share": [16384, 32768, 65536],
+    "cluster_min": [0, 2048, 8192, 16384, 32768, 65536, 131072],
+    "cluster_share": [0, 2048, 8192, 16384, 32768, 65536],
 }
 _INT_FIELDS = ("realclus", "dmpclus")
 _FLOAT_FIELDS = ("masa", "radio", "clusrx", "clusry", "clusrz", "msub", "rsub")
 
 
 def valid(p: dict) -> bool:
-    """tier1 <= tier2 <= cluster_min (the setters refuse tier2 < tier1)."""
-    return 0 < p["tier1"] <= p["tier2"] <= p["cluster_min"] and p["cluster_share"] > 0
+    """tier1 <= tier2 <= cluster_min (the setters refuse tier2 < tier1); a
+    cluster threshold or share of 0 is the library's rule."""
+    return (0 < p["tier1"] <= p["tier2"] and (p["cluster_min"] == 0 or p["tier2"] <= p["cluster_min"])
+            and p["cluster_share"] >= 0)
 
 
 def apply(lib, p: dict) -> None:
@@ -119,7 +127,7 @@ def same_catalogue(a: dict, b: dict, rtol: float = 1e-5) -> bool:
 
 
 def tune(timer, space: dict | None = None, start: dict | None = None, rounds: int = 2, verify=None):
-    """Coordinate descent over ``space`` from ``start`` (the defaults).
+    """Coordinate descent over ``space`` from ``start`` (``DEFAULTS``).
 
     timer(p) -> ms for a setting p; verify(p) -> bool, called once on the
     chosen setting when it differs from the start (the catalogue check): a
@@ -166,11 +174,11 @@ def tune_plan(plan, backend, with_subs: bool = True, reps: int = 3, space: dict 
     timer = device_timer(plan, backend, with_subs, reps)
     verify = None
     if check:
-        ref = catalogue_of(plan, backend, DEFAULTS, with_subs)
+        ref = catalogue_of(plan, backend, LIBRARY, with_subs)
 
         def verify(p):
             return same_catalogue(ref, catalogue_of(plan, backend, p, with_subs))
-    best, ms, trials = tune(timer, space, DEFAULTS, rounds, verify)
+    best, ms, trials = tune(timer, space, LIBRARY, rounds, verify)
     apply(backend.a, best)
     return best, ms, trials
 

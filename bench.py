@@ -13,8 +13,8 @@ subhaloes); inputs (4.3 GB of particles) are far larger than L2.
          host->device copy of the particles and device->host copy of the
          catalogue and IDs inside the timed region.
 Before the timed steps the size-tier thresholds of the per-halo kernels are
-tuned on the workload itself (asohf_b200/autotune.py; --no-tune keeps the
-defaults); the line names the setting used (launch_shape).
+tuned on the workload itself (asohf_b200/autotune.py; --no-tune leaves them
+to the library); the line names the setting used (launch_shape).
 Multi-GPU: the path does not exchange data, so every rank runs a replica
 on its own snapshot (weak scaling).
 
@@ -263,7 +263,7 @@ def main():
                     help="skip the end-to-end leg (profiling runs: only the device-timed steps)")
     ap.add_argument("--no-grid", action="store_true", help="skip the grid halo finder leg")
     ap.add_argument("--no-tune", action="store_true",
-                    help="keep the default size-tier thresholds (no launch-shape tuning before the timed steps)")
+                    help="leave the size-tier thresholds to the library (no launch-shape tuning before the timed steps)")
     ap.add_argument("--layer-only", action="store_true",
                     help="only the deposit+Poisson layer leg (profiling runs of its kernels)")
     args = ap.parse_args()
@@ -322,8 +322,8 @@ def main():
     b.a.set_stream(torch.cuda.current_stream().cuda_stream)
     # the size-tier thresholds: tuned on this workload before the timed steps
     # (coordinate descent, 2 timed runs per setting, the chosen setting's
-    # catalogue checked against the defaults'), or the defaults
-    launch = {"setting": dict(autotune.DEFAULTS), "tuned": False}
+    # catalogue checked against the untouched library's), or the library's own
+    launch = {"setting": dict(autotune.LIBRARY), "tuned": False}
     if not args.no_tune:
         best, ms_best, trials = autotune.tune_plan(plan, b, with_subs=with_subs, reps=2, rounds=1)
         launch = {"setting": best, "tuned": True, "settings_timed": len(trials),
