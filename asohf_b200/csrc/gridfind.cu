@@ -174,11 +174,18 @@ __global__ void k_grid_peaks(const float* __restrict__ u, int nx, float thr, uns
 // warp each.  The warp walks a shell's box 32 cells at a time in (K, J, I)
 // order, appends the cells inside the shell to a buffer in shared memory, and
 // lanes 0-5 then add one sum each in that order (REAL*4, the reference's
-// chain of additions).  Bound by that chain and the box walk of the largest
-// halo.  The chunks of a 128^3 grid take 0.25 ms with the replay below, 0.96 ms
-// with a row of the box at a time, every sum on every lane and two shuffles a
-// cell.
+// chain of additions).  Bound by that chain and the walk of the largest halo.
+// The chunks of a 128^3 grid take 0.25 ms with the replay below, 0.96 ms with a
+// row of the box at a time, every sum on every lane and two shuffles a cell.
+//
+// A box of wx cells a side holds wx^3 cells, its shell some 15 wx^2 with the
+// margins of row_runs: wide boxes are walked by rows, 32 rows' runs end to end.
+// Whole calls with haloes of 13, 21, 30, 62, 100 and 155 cells: 1.4, 3.3, 7.2,
+// 48, 182 and 575 ms; 2.2, 6.9, 18, 143, 568 and 1903 ms with every cell of the
+// box; with rows from 24 cells on the first two 1.8 and 3.7 ms.  Haloes of 2 to 6
+// cells take the same time both ways.
 constexpr int GF_BUF = 64;  // buffered cells of a warp: fewer than 32 left over, 32 appended
+constexpr int GF_ROWS = 16;  // cells a box row from which only the rows and cells that can meet the shell are walked
 __global__ void __launch_bounds__(128) k_grid_grow(GridIn G, GridChunk C, const uint8_t* __restrict__ conta) {
   __shared__ float s_term[4][6][GF_BUF];
   const unsigned FULL = 0xffffffffu;
@@ -216,15 +223,13 @@ __global__ void __launch_bounds__(128) k_grid_grow(GridIn G, GridChunk C, const 
     if (lane == 3) sum = __fadd_rn(yc, r_ext);
     if (lane == 4) sum = __fadd_rn(zc, r_ext);
     const int wx = hx - lx + 1, wy = hy - ly + 1;
-    const int rows = 32 / max(wx, 1), rest = 32 - rows * max(wx, 1);  // 32 cells on: rows down, rest along
-    int i = lx + lane % max(wx, 1), j = ly + lane / max(wx, 1), k = lz;
-    if (wx < 1 || wy < 1) k = hz + 1;
     int n = 0;
-    while (__any_sync(FULL, k <= hz)) {
-      while (j > hy && k <= hz) { j -= wy; k++; }
+    // a cell a lane, in (K, J, I) order: those inside the shell to the buffer,
+    // which is added as soon as it holds 32
+    auto take = [&](bool live, int i, int j, int k) {
       bool in = false;
       float rxi = 0.0f, ryj = 0.0f, rzk = 0.0f;
-      if (k <= hz) {
+      if (live) {
         rxi = G.radx[i];
         ryj = G.radx[j];
         rzk = G.radx[k];
@@ -255,9 +260,45 @@ __global__ void __launch_bounds__(128) k_grid_grow(GridIn G, GridChunk C, const 
         }
         __syncwarp();
       }
-      i += rest;
-      j += rows;
-      if (i > hx) { i -= wx; j++; }
+    };
+    if (wx >= 1 && wx < GF_ROWS && wy >= 1) {  // every cell of the box, 32 on: rows down, rest along
+      const int rows = 32 / wx, rest = 32 - rows * wx;
+      int i = lx + lane % wx, j = ly + lane / wx, k = lz;
+      while (__any_sync(FULL, k <= hz)) {
+        while (j > hy && k <= hz) { j -= wy; k++; }
+        take(k <= hz, i, j, k);
+        i += rest;
+        j += rows;
+        if (i > hx) { i -= wx; j++; }
+      }
+    } else if (wx >= GF_ROWS && wy >= 1) {  // 32 rows of the box at a time: the cells of those the shell can meet, 32 on
+      const float o2m = __fmul_rn(__fmul_rn(r_ext, r_ext), 1.0001f);
+      int j = ly + lane % wy, k = lz + lane / wy;
+      while (__any_sync(FULL, k <= hz)) {
+        int a0 = 1, a1 = 0, b0 = 1, b1 = 0;
+        if (k <= hz) {
+          const float ddy = __fsub_rn(G.radx[j], yc), ddz = __fsub_rn(G.radx[k], zc);
+          const float s2 = __fadd_rn(__fmul_rn(ddy, ddy), __fmul_rn(ddz, ddz));
+          if (!(s2 > o2m)) row_runs(G, xc, s2, r_int, r_ext, lx, hx, &a0, &a1, &b0, &b1);
+        }
+        const int na = max(a1 - a0 + 1, 0), len = na + max(b1 - b0 + 1, 0);
+        int end = len;  // cells of the rows up to the lane's
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(FULL, end, o);
+          if (lane >= o) end += v;
+        }
+        const int total = __shfl_sync(FULL, end, 31);
+        for (int c0 = 0; c0 < total; c0 += 32) {
+          const int c = c0 + lane;
+          int row = 0;  // the first row whose end lies past c
+          for (int o = 16; o > 0; o >>= 1)
+            if (__shfl_sync(FULL, end, row + o - 1) <= c) row += o;
+          const int at = c - __shfl_sync(FULL, end - len, row), ra = __shfl_sync(FULL, na, row);
+          const int ia = __shfl_sync(FULL, a0, row) + at, ib = __shfl_sync(FULL, b0, row) + at - ra;
+          take(c < total, at < ra ? ia : ib, __shfl_sync(FULL, j, row), __shfl_sync(FULL, k, row));
+        }
+        for (j += 32; j > hy; j -= wy) k++;
+      }
     }
     for (int q = 0; q < n; q++) sum = __fadd_rn(sum, mine[q]);
     __syncwarp();
