@@ -28,6 +28,7 @@ int tsc_base_batched_f32(asohf_ctx* c, int nx, float xl, float dx, const float* 
 int tsc_base_batched_f64(asohf_ctx* c, int nx, float xl, float dx, const float* dradx, int batch,
                          int64_t n_per, const float* x, const float* y, const float* z,
                          const float* m, float denbas, double* acc, float* rho);
+size_t tsc_base_f64_bytes(int64_t n_per, int64_t g);
 
 #define ASOHF_CUFFT(call)                                                        \
   do {                                                                           \
@@ -257,11 +258,11 @@ __device__ __forceinline__ uint32_t spread3(uint32_t v) {
   return v;
 }
 
-// Small sets deposit in input order into float64 sums, 27 atomics a particle,
-// rounded in one more pass: the launches of the sort cost more than the
-// atomics' contention (to about 180000 particles) and than clearing and
-// rounding the float64 grid (to 4M cells).  (In float32 the unsorted sums of a
-// crowded cell were up to five times further off than the sorted ones.)
+// Small sets deposit in input order into float64 sums (k_tsc_base_groups),
+// rounded in one more pass: to 163840 particles and 4M cells that takes less than
+// the launches of the sort, also where all of them crowd in a few cells.  (In
+// float32 the unsorted sums of a crowded cell were up to five times further off
+// than the sorted ones.)
 #define LAYER_SMALL_N (5 << 15)
 #define LAYER_SMALL_G (1 << 22)
 
@@ -440,7 +441,7 @@ extern "C" int asohf_tsc_poisson_forward(asohf_ctx* c, int nx, float lado0, floa
   const bool small = ntot <= LAYER_SMALL_N && g <= LAYER_SMALL_G;
   const bool sorted = !small && layer_sortable(nx, batch, ntot);
   ASOHF_CHECK(arena_reserve(c, poisson_bytes(nx, batch) + (sorted ? layer_sort_bytes(nx, batch, ntot) : 0) +
-                                   (small ? 8 * (size_t)g : 0) + 1024));
+                                   (small ? tsc_base_f64_bytes(n_per, g) : 0) + 1024));
   const float* dradx;
   ASOHF_CHECK(radx_device(c, nx, radx, &dradx));
   if (!small) ASOHF_CUDA(cudaMemsetAsync(rho, 0, 4 * g, c->stream));
@@ -449,9 +450,8 @@ extern "C" int asohf_tsc_poisson_forward(asohf_ctx* c, int nx, float lado0, floa
   float denbas = dx * dx * dx * rote * (rete * rete * rete);
   const float xl = -lado0 / 2.0f;
   if (small) {
-    double* acc = (double*)arena_alloc(c, 8 * (size_t)g);
+    double* acc = (double*)arena_alloc(c, tsc_base_f64_bytes(n_per, g));
     if (!acc) return ASOHF_ERR_CAPACITY;
-    ASOHF_CUDA(cudaMemsetAsync(acc, 0, 8 * g, c->stream));
     ASOHF_CHECK(tsc_base_batched_f64(c, nx, xl, dx, dradx, batch, n_per, x, y, z, m, denbas, acc, rho));
   } else if (sorted) {
     LayerSort s;
