@@ -2287,6 +2287,13 @@ __global__ void k_tsc_finish(DevMesh M, const int32_t* __restrict__ multi, const
   }
 }
 
+// Without patches a store of up to this many particles deposits in its own
+// order: the bins cost more than they save (32768 particles on 64^3 0.054 and
+// 0.13 ms, 2.1M on 128^3 0.31 and 0.45, on 256^3 0.57 and 0.62; 6M on 128^3 0.74
+// and 0.87, but 1.7 and 0.72, 3.5 and 0.79 where they crowd; 16.8M on 256^3 3.7
+// and 3.1).
+#define TSC_DIRECT_N (1ll << 21)
+
 extern "C" int asohf_interpolate_density_tsc(asohf_ctx* c, int nx, float lado0, float dx,
                                              const float* radx, float rote, float rete,
                                              const asohf_mesh* mesh, float* u1, float* u11,
@@ -2300,22 +2307,31 @@ extern "C" int asohf_interpolate_density_tsc(asohf_ctx* c, int nx, float lado0, 
   int np = 0;
   for (int ir = 1; ir <= nl; ir++) np += mesh->npatch[ir];
   if (np > 0 && !u11) return ASOHF_ERR_INVALID;
-  // bins of 2^3 base cells, particles within a bin by eighths of the cell:
-  // the base grid's cells and the patches' cells to level 2 stay together
-  const int bw = 2, sub = 3, nunits = TSLAB * np;
-  size_t need = 8 * g + 4 * g + 4 * (size_t)np * NA * NA * NA + 4 * (nx + 2) + 16 * n + 32 * (size_t)np +
-                unit_list_bytes(nunits) + bins_bytes(n, lado0, dx, bw, sub) + 16384;
+  // bins of 2^3 base cells, particles within a bin by eighths of it (its halves,
+  // the base cells, without patches): the base grid's cells and the patches'
+  // cells to level 2 stay together
+  const int bw = 2, sub = np ? 3 : 1, nunits = TSLAB * np;
+  const bool direct = np == 0 && n <= TSC_DIRECT_N && g < (1ll << 31);
+  const int copies = direct ? base_copies(n, g) : 1;
+  size_t need = 8 * g * copies + 4 * g + 4 * (size_t)np * NA * NA * NA + 4 * (nx + 2) + 32 * (size_t)np + 16384 +
+                (direct ? 0 : 16 * n + unit_list_bytes(nunits) + bins_bytes(n, lado0, dx, bw, sub));
   ASOHF_CHECK(arena_reserve(c, need));
   float* dradx = upload_floats(c, radx, nx + 2);
-  double* acc = (double*)arena_alloc(c, 8 * g);
-  float4* bp = (float4*)arena_alloc(c, 16 * n + 16);
+  double* acc = (double*)arena_alloc(c, 8 * g * copies);
+  float4* bp = direct ? nullptr : (float4*)arena_alloc(c, 16 * n + 16);
   float* du1;
   ASOHF_CHECK(stage_out(c, u1, 4 * g, on_device, &du1));
-  if (!dradx || !acc || !bp) return ASOHF_ERR_CAPACITY;
-  ASOHF_CUDA(cudaMemsetAsync(acc, 0, 8 * g, c->stream));
+  if (!dradx || !acc || (!direct && !bp)) return ASOHF_ERR_CAPACITY;
+  ASOHF_CUDA(cudaMemsetAsync(acc, 0, 8 * g * copies, c->stream));
   float xl = -lado0 / 2.0f;
   Bins B;
-  if (n > 0) {
+  if (n > 0 && direct) {
+    int kt_ = ktime_begin(c, "tsc_base");
+    k_tsc_base_groups<<<grid_for(n, TG_BLOCK, c->num_sms * 16), TG_BLOCK, 0, c->stream>>>(
+        c->p.x, c->p.y, c->p.z, c->p.m, n, 1, nx, xl, dx, dradx, 1.0f, copies, acc);
+    ktime_end(c, kt_);
+    c->launches++;
+  } else if (n > 0) {
     ASOHF_CHECK(build_bins(c, lado0, dx, bw, &B, DAlloc{nullptr, false}, sub));
     int kt_ = ktime_begin(c, "tsc_base");
     k_bin_stage<<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(
@@ -2327,7 +2343,7 @@ extern "C" int asohf_interpolate_density_tsc(asohf_ctx* c, int nx, float lado0, 
     c->launches += 2;
   }
   float denbas = dx * dx * dx * rote * (rete * rete * rete);
-  k_finish_f64<<<grid_for(g, 256), 256, 0, c->stream>>>(acc, g, denbas, du1);
+  k_finish_copies<<<grid_for(g, 256), 256, 0, c->stream>>>(acc, g, copies, denbas, du1);
   c->launches++;
   ASOHF_CUDA(cudaGetLastError());
   if (!on_device) ASOHF_CUDA(cudaMemcpyAsync(u1, du1, 4 * g, cudaMemcpyDeviceToHost, c->stream));
