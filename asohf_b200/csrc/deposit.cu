@@ -565,14 +565,23 @@ __global__ void k_finish_f64(const double* __restrict__ acc, int64_t g, float de
 struct Bins {
   int nb;          // bins per axis
   float xl, bsz;   // origin and bin size
+  float eps;       // in bins: a particle this little below a bin's lower face is in it
   int32_t* start;  // nb^3+1
   int32_t* idx;    // particle indices grouped by bin
 };
 
-__device__ __forceinline__ int bin_of(float v, float xl, float bsz, int nb) {
-  int b = (int)floorf((v - xl) / bsz);
+// A range's lower bound and the reference's own INT((v - patch corner) / cell)
+// round differently, so a particle may belong to a unit though its coordinate
+// lies a few spacings below the bound: with the faces on a common grid that is a
+// few spacings below a bin.  Particles are therefore binned eps = nb 2^-20 up
+// (the roundings add to less than 10 nb 2^-24), and a range runs from the bin of
+// its lower bound to the bin of its upper bound moved up likewise.
+__device__ __forceinline__ int bin_clamp(float t, int nb) {
+  const int b = (int)floorf(t);
   return b < 0 ? 0 : (b >= nb ? nb - 1 : b);
 }
+__device__ __forceinline__ int bin_lo(const Bins& B, float v) { return bin_clamp((v - B.xl) / B.bsz, B.nb); }
+__device__ __forceinline__ int bin_hi(const Bins& B, float v) { return bin_clamp((v - B.xl) / B.bsz + B.eps, B.nb); }
 
 // Sort key of a particle: its bin, then `sub` bits per axis of its place
 // inside the bin, interleaved (0: input order within a bin).  With sub bits
@@ -582,9 +591,8 @@ __device__ __forceinline__ uint32_t bin_key(const Bins& B, float x, float y, flo
   const float v[3] = {x, y, z};
   uint32_t b[3], low = 0;
   for (int a = 0; a < 3; a++) {
-    const float t = (v[a] - B.xl) / B.bsz;
-    const int c = (int)floorf(t);
-    b[a] = (uint32_t)(c < 0 ? 0 : (c >= B.nb ? B.nb - 1 : c));
+    const float t = (v[a] - B.xl) / B.bsz + B.eps;
+    b[a] = (uint32_t)bin_clamp(t, B.nb);
     if (sub) {
       const int m = 1 << sub, q = (int)((t - (float)b[a]) * (float)m);
       const uint32_t u = (uint32_t)(q < 0 ? 0 : (q >= m ? m - 1 : q));
@@ -672,6 +680,7 @@ static int build_bins(asohf_ctx* c, float lado0, float dx, int bw, Bins* B, DAll
   B->nb = nb;
   B->xl = -lado0 / 2.0f;
   B->bsz = lado0 / (float)nb;
+  B->eps = ldexpf((float)nb, -20);
   uint32_t* k0 = (uint32_t*)arena_alloc(c, 4 * n + 4);
   uint32_t* k1 = (uint32_t*)arena_alloc(c, 4 * n + 4);
   int32_t* v0 = (int32_t*)arena_alloc(c, 4 * n + 4);
@@ -901,13 +910,13 @@ __device__ __forceinline__ void unit_geo(const DevMesh& M, const Bins& B, const 
   g.pxr = (g.xlfix + (float)g.n1 * g.dxpa) + dx;
   g.pyr = (g.ylfix + (float)g.n2 * g.dxpa) + dx;
   g.pzr = (g.zlfix + (float)g.n3 * g.dxpa) + dx;
-  g.bx0 = bin_of(g.pxl, B.xl, B.bsz, B.nb); g.bx1 = bin_of(g.pxr, B.xl, B.bsz, B.nb);
-  g.by0 = bin_of(g.pyl, B.xl, B.bsz, B.nb); g.by1 = bin_of(g.pyr, B.xl, B.bsz, B.nb);
+  g.bx0 = bin_lo(B, g.pxl); g.bx1 = bin_hi(B, g.pxr);
+  g.by0 = bin_lo(B, g.pyl); g.by1 = bin_hi(B, g.pyr);
   // a cloud reaches at most 2^ir cells = DX from its host cell: planes
   // zlo..zhi take hosts with z in [zlfix + (zlo-1) dxpa - DX, zlfix + zhi dxpa + DX]
   float za = fmaxf(g.pzl, (g.zlfix + (float)(g.zlo - 1) * g.dxpa) - dx);
   float zb = fminf(g.pzr, (g.zlfix + (float)g.zhi * g.dxpa) + dx);
-  g.bz0 = bin_of(za, B.xl, B.bsz, B.nb); g.bz1 = bin_of(zb, B.xl, B.bsz, B.nb);
+  g.bz0 = bin_lo(B, za); g.bz1 = bin_hi(B, zb);
   g.nby = g.by1 - g.by0 + 1;
   g.rows = (g.zlo > g.zhi) ? 0 : g.nby * (g.bz1 - g.bz0 + 1);
 }
@@ -2167,13 +2176,13 @@ __device__ __forceinline__ void tsc_unit_geo(const DevMesh& M, const Bins& B, in
   g.pxr = g.pxl + (float)(g.n1 + 2) * g.dxpa;
   g.pyr = g.pyl + (float)(g.n2 + 2) * g.dxpa;
   g.pzr = g.pzl + (float)(g.n3 + 2) * g.dxpa;
-  g.bx0 = bin_of(g.pxl, B.xl, B.bsz, B.nb); g.bx1 = bin_of(g.pxr, B.xl, B.bsz, B.nb);
-  g.by0 = bin_of(g.pyl, B.xl, B.bsz, B.nb); g.by1 = bin_of(g.pyr, B.xl, B.bsz, B.nb);
+  g.bx0 = bin_lo(B, g.pxl); g.bx1 = bin_hi(B, g.pxr);
+  g.by0 = bin_lo(B, g.pyl); g.by1 = bin_hi(B, g.pyr);
   // planes zlo..zhi take cells zlo-1..zhi+1, cell k from pzl + k dxpa; half a
   // cell more on each side for the rounding of the quotient
   const float za = fmaxf(g.pzl, g.pzl + ((float)g.zlo - 1.5f) * g.dxpa);
   const float zb = fminf(g.pzr, g.pzl + ((float)g.zhi + 2.5f) * g.dxpa);
-  g.bz0 = bin_of(za, B.xl, B.bsz, B.nb); g.bz1 = bin_of(zb, B.xl, B.bsz, B.nb);
+  g.bz0 = bin_lo(B, za); g.bz1 = bin_hi(B, zb);
   g.nby = g.by1 - g.by0 + 1;
   g.rows = (g.zlo > g.zhi) ? 0 : g.nby * (g.bz1 - g.bz0 + 1);
 }
@@ -2502,12 +2511,12 @@ __device__ __forceinline__ void mesh_unit_geo(const MeshPatches& M, const Bins& 
   g.ylfix = __fsub_rn(M.r[M.np + g.ip], M.dxpa);
   g.zlfix = __fsub_rn(M.r[2 * M.np + g.ip], M.dxpa);
   const float pad = 2.0f * M.dxpa;
-  g.bx0 = bin_of(g.xlfix - pad, B.xl, B.bsz, B.nb);
-  g.bx1 = bin_of(g.xlfix + (float)(g.n1 + 2) * M.dxpa, B.xl, B.bsz, B.nb);
-  g.by0 = bin_of(g.ylfix - pad, B.xl, B.bsz, B.nb);
-  g.by1 = bin_of(g.ylfix + (float)(g.n2 + 2) * M.dxpa, B.xl, B.bsz, B.nb);
-  g.bz0 = bin_of(g.zlfix + (float)(g.zlo - 2) * M.dxpa, B.xl, B.bsz, B.nb);
-  g.bz1 = bin_of(g.zlfix + (float)(g.zhi + 3) * M.dxpa, B.xl, B.bsz, B.nb);
+  g.bx0 = bin_lo(B, g.xlfix - pad);
+  g.bx1 = bin_hi(B, g.xlfix + (float)(g.n1 + 2) * M.dxpa);
+  g.by0 = bin_lo(B, g.ylfix - pad);
+  g.by1 = bin_hi(B, g.ylfix + (float)(g.n2 + 2) * M.dxpa);
+  g.bz0 = bin_lo(B, g.zlfix + (float)(g.zlo - 2) * M.dxpa);
+  g.bz1 = bin_hi(B, g.zlfix + (float)(g.zhi + 3) * M.dxpa);
   g.nby = g.by1 - g.by0 + 1;
   g.rows = g.zlo > g.zhi ? 0 : g.nby * (g.bz1 - g.bz0 + 1);
 }
