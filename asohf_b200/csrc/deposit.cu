@@ -874,13 +874,28 @@ k_base_stencil(const int32_t* __restrict__ cnt, int nx, Terms8 T, float denbas, 
 // Work unit: PZ z-planes of one patch.  A unit's candidates are the particles
 // of the bins that overlap the patch box extended by MAXKERNELEXT = DX
 // (grids.f:837-893), restricted in z to the unit's planes +- DX; they are split
-// into slices of PSLICE so that a dense unit is shared by several CTAs, whose
-// sums meet in a float64 scratch slab.
+// into slices so that a dense unit is shared by several CTAs, whose sums meet in
+// a float64 scratch slab.
 #define PZ 4              // z planes per unit
 #define PZ_BLOCK 256
 #define NSLAB (NA / PZ)
-#define PSLICE 24576      // candidates per work item: counts of a slice fit 16 bits (of 8192, 16384, 24576 and
-                          // 32768, the equal-mass kernel measured 17.5, 16.3, 15.9, 15.7 ms at 384^3)
+// Slices are cut by work: the candidates, weighted by the width of their clouds
+// in a sample of the unit's.  A slice holds the share that gives `items` of them
+// an SM, between lo and hi, or a twelfth of an SM's work where that is more.
+// Large slices cost least where every CTA has many units to take (the equal-mass
+// kernel at 384^3 with 8192, 16384, 24576 and 32768: 17.5, 16.3, 15.9, 15.7 ms),
+// small ones spread few units, or few with many wide clouds: DENSITY of 262144
+// particles on 299 patches to level 3 takes 0.38 ms with their species (0.44 with
+// slices of 24576) and 1.7 with one species (8.1); 2.1M on 2207 patches 1.43
+// (1.42) and 7.4 (10.7); 56.6M on 12012 25.6 (25.4).  Weights of 1, 8, 100 and 100
+// cut ordinary units too often (2.1M to level 6 1.82 ms, 1.77 so).
+struct SliceRule {
+  int items, lo, hi;  // hi also bounds the candidates: the equal-mass kernel counts a slice's in 16 bits
+  int w[4];           // weight of a cloud of level 1 or less, 2, 3, 4 or more
+};
+static const SliceRule kSliceEq{3, 8192, 24576, {1, 3, 6, 6}}, kSliceAny{6, 2048, 24576, {1, 2, 4, 13}},
+    kSliceUnits{6, 2048, 24576, {1, 1, 1, 1}};
+#define SLICE_MIN 256  // candidates
 #define PROWS 128         // bin rows staged in shared memory at a time
 #define AROW (NA + 5)     // accumulator row stride (doubles): rows shifted by 5 banks pairs
 #define APLANE (NA * AROW)
@@ -929,35 +944,51 @@ __device__ __forceinline__ void row_range(const Bins& B, const UnitGeo& g, int r
   *len = b - a;
 }
 
-// Candidates of a unit (one warp per unit), as a sort key that puts the
-// largest count first.
-__device__ __forceinline__ void unit_count(const Bins& B, const UnitGeo& g, int u, int lane, uint32_t* key,
-                                           int32_t* unit) {
-  long long s = 0;
+// Candidates of a unit (one warp per unit) and its work, candidates times their
+// weights in a sample of two a row, in sixteenths as a sort key that puts the
+// largest first.
+template <typename F>
+__device__ __forceinline__ void unit_count(const Bins& B, const UnitGeo& g, int u, int lane, F weight, uint32_t* cnt,
+                                           uint32_t* key, int32_t* unit, int32_t* nm) {
+  long long s = 0, w = 0;
   for (int r = lane; r < g.rows; r += 32) {
     int lo, len;
     row_range(B, g, r, &lo, &len);
     s += len;
+    if (len > 0) w += ((long long)len * (weight(lo + len / 4) + weight(lo + (int)(3ll * len / 4))) + 1) / 2;
   }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_down_sync(0xffffffffu, s, o);
+    w += __shfl_down_sync(0xffffffffu, w, o);
+  }
   if (lane == 0) {
-    key[u] = ~(uint32_t)(s < 0xffffffffll ? s : 0xffffffffll);
+    w = (w + 15) / 16;
+    cnt[u] = (uint32_t)(s < 0xffffffffll ? s : 0xffffffffll);
+    key[u] = ~(uint32_t)(w < 0xffffffffll ? w : 0xffffffffll);
     unit[u] = u;
+    if (u == 0) *nm = 0;
   }
 }
 
+// P holds the species in w, or S does (P null).
 __global__ void k_patch_unit_counts(DevMesh M, Bins B, const int32_t* __restrict__ order, int nunits, float dx,
-                                    uint32_t* __restrict__ key, int32_t* __restrict__ unit) {
+                                    const float4* __restrict__ P, const uint8_t* __restrict__ S, SliceRule R,
+                                    uint32_t* __restrict__ cnt, uint32_t* __restrict__ key,
+                                    int32_t* __restrict__ unit, int32_t* __restrict__ nm) {
   int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (u >= nunits) return;
   UnitGeo g;
   unit_geo(M, B, order, u, dx, g);
-  unit_count(B, g, u, lane, key, unit);
+  auto weight = [&](int e) {
+    const int s = P ? __float_as_int(P[e].w) : (int)S[e], l = s == 255 ? 0 : g.ir - s;
+    return l <= 1 ? R.w[0] : (l == 2 ? R.w[1] : (l == 3 ? R.w[2] : R.w[3]));
+  };
+  unit_count(B, g, u, lane, weight, cnt, key, unit, nm);
 }
 
 struct PatchWork {
   const int2* items;         // (unit, slice)
-  const int32_t* scratch_of; // per unit: scratch slab index, -1 for single-slice units
+  const int2* unit;          // per unit: scratch slab index (-1: one slice), candidates of a slice
   double* scratch;           // the unit's cells in float64, per multi-slice unit
 };
 
@@ -996,16 +1027,17 @@ __device__ __forceinline__ int find_row(const int* s_pre, int nr, int v) {
 }
 
 // Work items of a patch deposit, built on the device: the units in order of
-// falling candidate count, each cut into slices of PSLICE.  The host reads two
-// numbers (items, units with several slices) to size the buffers.  (Counts to
+// falling work, each cut into slices.  The host reads two numbers (items, the last
+// unit with several slices) to size the buffers.  (Counts to
 // the host, sorted there and the lists sent back took 1.6 ms of the 37 ms of
 // 12012 patches at 384^3; this takes under 0.1 ms.)
 struct UnitList {
   int nunits = 0, nitems = 0, nmulti = 0;
-  uint32_t *key = nullptr, *key2 = nullptr;  // ~count, by unit and sorted
+  uint32_t* cnt = nullptr;                   // candidates, by unit
+  uint32_t *key = nullptr, *key2 = nullptr;  // ~work, by unit and sorted
   int32_t *unit = nullptr, *ord = nullptr;
   int32_t *ns = nullptr, *off = nullptr;     // slices of each sorted unit, and the sum before it
-  int32_t* nm = nullptr;
+  int32_t* nm = nullptr;                     // the last sorted unit with several, plus 1
   void* tmp = nullptr;
   size_t sort_b = 0, scan_b = 0;
 };
@@ -1020,12 +1052,13 @@ static void unit_list_temp(int nunits, size_t* sort_b, size_t* scan_b) {
 static size_t unit_list_bytes(int nunits) {
   size_t a, b;
   unit_list_temp(nunits, &a, &b);
-  return 32 * (size_t)nunits + (a > b ? a : b) + 16 * 256;
+  return 36 * (size_t)nunits + (a > b ? a : b) + 16 * 256;
 }
 
 static int unit_list_begin(asohf_ctx* c, int nunits, UnitList* U) {
   U->nunits = nunits;
   const size_t b = 4 * (size_t)nunits + 4;
+  U->cnt = (uint32_t*)arena_alloc(c, b);
   U->key = (uint32_t*)arena_alloc(c, b);
   U->key2 = (uint32_t*)arena_alloc(c, b);
   U->unit = (int32_t*)arena_alloc(c, b);
@@ -1035,32 +1068,47 @@ static int unit_list_begin(asohf_ctx* c, int nunits, UnitList* U) {
   U->nm = (int32_t*)arena_alloc(c, 4);
   unit_list_temp(nunits, &U->sort_b, &U->scan_b);
   U->tmp = arena_alloc(c, U->sort_b > U->scan_b ? U->sort_b : U->scan_b);
-  return U->key && U->key2 && U->unit && U->ord && U->ns && U->off && U->nm && U->tmp ? ASOHF_OK
-                                                                                      : ASOHF_ERR_CAPACITY;
+  return U->cnt && U->key && U->key2 && U->unit && U->ord && U->ns && U->off && U->nm && U->tmp
+             ? ASOHF_OK
+             : ASOHF_ERR_CAPACITY;
 }
 
-__device__ __forceinline__ int unit_slices(uint32_t key) {
-  const uint32_t cnt = ~key;
-  return cnt > PSLICE ? (int)((cnt - 1) / PSLICE) + 1 : 1;
-}
-
-__global__ void k_unit_slices(const uint32_t* __restrict__ key, int n, int32_t* __restrict__ ns,
+// Slices of the sorted units (256 threads).  Every CTA forms the share of work
+// from the sum over all units: over up to 1024 of them, else over 1024 evenly
+// spaced ones (the work falls steadily) times their distance.
+__global__ void k_unit_slices(const uint32_t* __restrict__ key, const int32_t* __restrict__ ord,
+                              const uint32_t* __restrict__ cnt, int n, int sms, SliceRule R, int32_t* __restrict__ ns,
                               int32_t* __restrict__ nm) {
+  __shared__ double s_sum[8];
+  const int step = n > 1024 ? n / 1024 : 1;
+  double sum = 0.0;
+  for (int64_t q = (int64_t)threadIdx.x * step; q < n; q += 256 * (int64_t)step) sum += (double)(~key[q]);
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  sum = 0.0;
+  for (int w = 0; w < 8; w++) sum += s_sum[w];
+  const double sm = 16.0 * sum * step / sms;  // an SM's work
+  const double share = fmax(fmin(fmax(sm / R.items, (double)R.lo), (double)R.hi), sm / 12.0);
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r > n) return;
-  const int k = r < n ? unit_slices(key[r]) : 0;
+  int k = 0;
+  if (r < n) {
+    const uint32_t m = cnt[ord[r]];
+    const double most = fmax(1.0, (double)(m / SLICE_MIN));
+    k = (int)fmin(most, ceil(16.0 * (double)(~key[r]) / share));
+    k = max(max(k, 1), (int)((m + (uint64_t)R.hi - 1) / R.hi));
+  }
   ns[r] = k;
-  // counts fall with r: the units of several slices come first
-  if (r == 0 && k <= 1) *nm = 0;
-  if (k > 1 && (r == n - 1 || unit_slices(key[r + 1]) <= 1)) *nm = r + 1;
+  if (k > 1) atomicMax(nm, r + 1);
 }
 
-// After the counts: the sort, the slices and their sum; reads the two totals.
-static int unit_list_size(asohf_ctx* c, UnitList* U) {
+// After the counts: the sort, the slices and their sum; reads the totals.
+static int unit_list_size(asohf_ctx* c, UnitList* U, SliceRule R) {
   const int n = U->nunits;
   ASOHF_CUDA(cub::DeviceRadixSort::SortPairs(U->tmp, U->sort_b, U->key, U->key2, U->unit, U->ord, n, 0, 32,
                                              c->stream));
-  k_unit_slices<<<n / 256 + 1, 256, 0, c->stream>>>(U->key2, n, U->ns, U->nm);
+  k_unit_slices<<<n / 256 + 1, 256, 0, c->stream>>>(U->key2, U->ord, U->cnt, n, c->num_sms, R, U->ns, U->nm);
   ASOHF_CUDA(cub::DeviceScan::ExclusiveSum(U->tmp, U->scan_b, U->ns, U->off, n + 1, c->stream));
   c->launches++;
   int32_t h[2];
@@ -1076,19 +1124,20 @@ static size_t unit_work_bytes(const UnitList& U, int unit_cells) {
   return sizeof(int2) * (size_t)U.nitems + 4 * (size_t)U.nmulti + 8 * (size_t)unit_cells * U.nmulti + 4 * 256;
 }
 
+// multi: the unit of each scratch slab, -1 where the slab is not used.
 __global__ void k_unit_items(const int32_t* __restrict__ ord, const int32_t* __restrict__ ns,
-                             const int32_t* __restrict__ off, int n, int2* __restrict__ items,
-                             int32_t* __restrict__ scratch_of, int32_t* __restrict__ multi) {
+                             const int32_t* __restrict__ off, const uint32_t* __restrict__ cnt, int n, int nmulti,
+                             int2* __restrict__ items, int2* __restrict__ unit, int32_t* __restrict__ multi) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   const int u = ord[r], k = ns[r], o = off[r];
   for (int q = 0; q < k; q++) items[o + q] = make_int2(u, q);
-  scratch_of[u] = k > 1 ? r : -1;
-  if (k > 1) multi[r] = u;
+  unit[u] = make_int2(k > 1 ? r : -1, (int)((cnt[u] + (uint64_t)k - 1) / k));
+  if (r < nmulti) multi[r] = k > 1 ? u : -1;
 }
 
 // The items, scratch slabs (cleared) and slab indices, in buffers of the
-// caller's: `walloc` for what unit_work_bytes counts, `salloc` for 4 bytes a unit.
+// caller's: `walloc` for what unit_work_bytes counts, `salloc` for 8 bytes a unit.
 template <typename FW, typename FS>
 static int unit_list_fill(asohf_ctx* c, const UnitList& U, int unit_cells, FW walloc, FS salloc, PatchWork* W,
                           int32_t** multi) {
@@ -1096,13 +1145,14 @@ static int unit_list_fill(asohf_ctx* c, const UnitList& U, int unit_cells, FW wa
   *multi = (int32_t*)walloc(4 * (size_t)(U.nmulti > 0 ? U.nmulti : 1));
   const size_t sb = 8 * (size_t)unit_cells * U.nmulti;
   W->scratch = (double*)walloc(sb > 0 ? sb : 8);
-  int32_t* sof = (int32_t*)salloc(4 * (size_t)U.nunits);
-  if (!items || !*multi || !W->scratch || !sof) return ASOHF_ERR_CAPACITY;
+  int2* unit = (int2*)salloc(8 * (size_t)U.nunits);
+  if (!items || !*multi || !W->scratch || !unit) return ASOHF_ERR_CAPACITY;
   if (sb) ASOHF_CUDA(cudaMemsetAsync(W->scratch, 0, sb, c->stream));
-  k_unit_items<<<(U.nunits + 255) / 256, 256, 0, c->stream>>>(U.ord, U.ns, U.off, U.nunits, items, sof, *multi);
+  k_unit_items<<<(U.nunits + 255) / 256, 256, 0, c->stream>>>(U.ord, U.ns, U.off, U.cnt, U.nunits, U.nmulti, items,
+                                                                   unit, *multi);
   c->launches++;
   W->items = items;
-  W->scratch_of = sof;
+  W->unit = unit;
   return ASOHF_OK;
 }
 
@@ -1110,7 +1160,7 @@ static int unit_list_fill(asohf_ctx* c, const UnitList& U, int unit_cells, FW wa
 // unit's sums live in registers: lane i of warp w holds cells (i, 4w .. 4w+3,
 // every plane) in float64, so clouds are added without atomics.  Hosts of level
 // 0 and 1 (most hits) are counted, both levels in the halves of one word a cell
-// (a slice holds at most PSLICE hosts, so no half and no sum of counts
+// (a slice holds at most kSliceEq.hi hosts, so no half and no sum of counts
 // overflows), and spread by a stencil at the end: with a kernel symmetric in
 // each axis the (2r+1)^3 terms of a level take (r+1)^3 values t(|di|, |dj|,
 // |dk|), each formed once.  Wider clouds are listed by the scan and added by
@@ -1303,7 +1353,8 @@ k_density_patches_eq(DevMesh M, Bins B, const float4* __restrict__ P, const int3
       }
     }
   };
-  const int64_t v0 = (int64_t)it.y * PSLICE, v1 = v0 + PSLICE;
+  const int slice = W.unit[it.x].y;
+  const int64_t v0 = (int64_t)it.y * slice, v1 = v0 + slice;
   int64_t vbase = 0;
   for (int r0 = 0; r0 < g.rows; r0 += PROWS) {
     const int nr = min(PROWS, g.rows - r0);
@@ -1430,7 +1481,7 @@ k_density_patches_eq(DevMesh M, Bins B, const float4* __restrict__ P, const int3
       }
     }
   }
-  const int sidx = W.scratch_of[it.x];
+  const int sidx = W.unit[it.x].x;
   const float den = denbas_lev[g.ir];
 #pragma unroll
   for (int q = 0; q < 4; q++)
@@ -1477,7 +1528,8 @@ k_density_patches(DevMesh M, Bins B, const float4* __restrict__ P, const uint8_t
   if (threadIdx.x >= 1 && threadIdx.x <= NA) s_rcp[threadIdx.x] = 1.0f / (float)threadIdx.x;
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  const int64_t v0 = (int64_t)it.y * PSLICE, v1 = v0 + PSLICE;
+  const int slice = W.unit[it.x].y;
+  const int64_t v0 = (int64_t)it.y * slice, v1 = v0 + slice;
   int64_t vbase = 0;
   for (int r0 = 0; r0 < g.rows; r0 += PROWS) {
     int nr = min(PROWS, g.rows - r0);
@@ -1592,7 +1644,7 @@ k_density_patches(DevMesh M, Bins B, const float4* __restrict__ P, const uint8_t
     vbase += tot;
   }
   __syncthreads();
-  const int sidx = W.scratch_of[it.x];
+  const int sidx = W.unit[it.x].x;
   if (sidx < 0) {
     __syncthreads();
     const float den = denbas_lev[g.ir];
@@ -1617,6 +1669,7 @@ __global__ void k_patch_finish(DevMesh M, const int32_t* __restrict__ order, con
                                const double* __restrict__ scratch, float* __restrict__ u11,
                                const float* __restrict__ denbas_lev) {
   int u = multi[blockIdx.x];
+  if (u < 0) return;
   int ip = order[u / NSLAB], slab = u % NSLAB;
   int n1 = M.nx[ip], n2 = M.ny[ip], n3 = M.nz[ip];
   float den = denbas_lev[M.level[ip]];
@@ -1687,13 +1740,13 @@ extern "C" int asohf_density(asohf_ctx* c, int nx, float lado0, float dx, float 
   size_t need = 12 * g + (on_device ? 0 : 4 * g + 4 * (size_t)np * NA * NA * NA) +
                 16 * T2COPY + 96 * (size_t)np + 16384 +
                 (np ? std::max(bins_bytes(nall, lado0, dx, 2), bins_bytes(nall, lado0, dx, 2, 3)) + 17 * (size_t)nall + unit_list_bytes(NSLAB * np) +
-                          4 * NSLAB * (size_t)np : 0);
+                          8 * NSLAB * (size_t)np : 0);
   ASOHF_CHECK(arena_reserve(c, need));
   if (defer) {  // what the deferred kernels read: mesh, order, bins, staged particles, renorm dims
     const int nbw = (int)lrintf(lado0 / dx);
     const int64_t nb = (nbw + 1) / 2, nbin = nb * nb * nb;
     ASOHF_CHECK(dpool_reserve(c, 0, 16 * T2COPY + 4 * (ASOHF_NLEVELS + 1) + 48 * (size_t)np +
-                                        4 * (size_t)(nbin + 1) + 17 * (size_t)nall + 4 * NSLAB * (size_t)np +
+                                        4 * (size_t)(nbin + 1) + 17 * (size_t)nall + 8 * NSLAB * (size_t)np +
                                         16 * 256));
   }
   const float* hk;
@@ -1813,11 +1866,13 @@ extern "C" int asohf_density(asohf_ctx* c, int nx, float lado0, float dx, float 
       const int nunits = NSLAB * np;
       UnitList U;
       ASOHF_CHECK(unit_list_begin(c, nunits, &U));
-      k_patch_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, order, nunits, dx, U.key, U.unit);
+      const SliceRule R = pd_eq ? kSliceEq : kSliceAny;
+      k_patch_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, order, nunits, dx, pd_eq ? bp : nullptr, bs, R,
+                                                                   U.cnt, U.key, U.unit, U.nm);
       c->launches++;
-      // work list: slices of PSLICE candidates, the densest units first; in
+      // work list: slices of the candidates, the densest units first; in
       // the segment buffers, or density pool 1 when deferred
-      ASOHF_CHECK(unit_list_size(c, &U));
+      ASOHF_CHECK(unit_list_size(c, &U, R));
       const size_t wbytes = unit_work_bytes(U, NA * NA * PZ);
       ASOHF_CHECK(defer ? dpool_reserve(c, 1, wbytes) : seg_reserve(c, wbytes));
       PatchWork W;
@@ -2207,7 +2262,8 @@ k_tsc_patches(DevMesh M, Bins B, const float4* __restrict__ P, PatchWork W, floa
   float* w = s_w[threadIdx.x >> 5];
   const int i3 = lane % 3, j3 = (lane / 3) % 3, k3 = min(lane / 9, 2);
   const float rx = M.rx[g.ip], ry = M.ry[g.ip], rz = M.rz[g.ip];
-  const int64_t v0 = (int64_t)it.y * PSLICE, v1 = v0 + PSLICE;
+  const int slice = W.unit[it.x].y;
+  const int64_t v0 = (int64_t)it.y * slice, v1 = v0 + slice;
   int64_t vbase = 0;
   for (int r0 = 0; r0 < g.rows; r0 += PROWS) {
     const int nr = min(PROWS, g.rows - r0);
@@ -2261,7 +2317,7 @@ k_tsc_patches(DevMesh M, Bins B, const float4* __restrict__ P, PatchWork W, floa
     vbase += tot;
   }
   __syncthreads();
-  const int sidx = W.scratch_of[it.x];
+  const int sidx = W.unit[it.x].x;
   const float den = denbas_lev[g.ir];
   for (int q = threadIdx.x; q < NA * NA * TZ; q += blockDim.x) {
     const int i = q % NA, j = (q / NA) % NA, k = q / (NA * NA);
@@ -2273,19 +2329,20 @@ k_tsc_patches(DevMesh M, Bins B, const float4* __restrict__ P, PatchWork W, floa
   }
 }
 
-__global__ void k_tsc_unit_counts(DevMesh M, Bins B, int nunits, float dx, uint32_t* __restrict__ key,
-                                  int32_t* __restrict__ unit) {
+__global__ void k_tsc_unit_counts(DevMesh M, Bins B, int nunits, float dx, uint32_t* __restrict__ cnt,
+                                  uint32_t* __restrict__ key, int32_t* __restrict__ unit, int32_t* __restrict__ nm) {
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (u >= nunits) return;
   UnitGeo g;
   tsc_unit_geo(M, B, u, dx, g);
-  unit_count(B, g, u, lane, key, unit);
+  unit_count(B, g, u, lane, [](int) { return 1; }, cnt, key, unit, nm);
 }
 
 // Units shared by several slices: the summed scratch slab to U11.
 __global__ void k_tsc_finish(DevMesh M, const int32_t* __restrict__ multi, const double* __restrict__ scratch,
                              float* __restrict__ u11, const float* __restrict__ denbas_lev) {
   const int u = multi[blockIdx.x], ip = u / TSLAB, slab = u % TSLAB;
+  if (u < 0) return;
   const int n1 = M.nx[ip], n2 = M.ny[ip], n3 = M.nz[ip];
   const float den = denbas_lev[M.level[ip]];
   const double* sc = scratch + (size_t)blockIdx.x * NA * NA * TZ;
@@ -2322,7 +2379,7 @@ extern "C" int asohf_interpolate_density_tsc(asohf_ctx* c, int nx, float lado0, 
   const int bw = 2, sub = np ? 3 : 1, nunits = TSLAB * np;
   const bool direct = np == 0 && n <= TSC_DIRECT_N && g < (1ll << 31);
   const int copies = direct ? base_copies(n, g) : 1;
-  size_t need = 8 * g * copies + 4 * g + 4 * (size_t)np * NA * NA * NA + 4 * (nx + 2) + 32 * (size_t)np + 16384 +
+  size_t need = 8 * g * copies + 4 * g + 4 * (size_t)np * NA * NA * NA + 4 * (nx + 2) + 64 * (size_t)np + 16384 +
                 (direct ? 0 : 16 * n + unit_list_bytes(nunits) + bins_bytes(n, lado0, dx, bw, sub));
   ASOHF_CHECK(arena_reserve(c, need));
   float* dradx = upload_floats(c, radx, nx + 2);
@@ -2371,9 +2428,9 @@ extern "C" int asohf_interpolate_density_tsc(asohf_ctx* c, int nx, float lado0, 
       if (!dden) return ASOHF_ERR_CAPACITY;
       UnitList U;
       ASOHF_CHECK(unit_list_begin(c, nunits, &U));
-      k_tsc_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, nunits, dx, U.key, U.unit);
+      k_tsc_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, nunits, dx, U.cnt, U.key, U.unit, U.nm);
       c->launches++;
-      ASOHF_CHECK(unit_list_size(c, &U));
+      ASOHF_CHECK(unit_list_size(c, &U, kSliceUnits));
       ASOHF_CHECK(seg_reserve(c, unit_work_bytes(U, NA * NA * TZ)));
       PatchWork W;
       int32_t* multi;
@@ -2521,13 +2578,13 @@ __device__ __forceinline__ void mesh_unit_geo(const MeshPatches& M, const Bins& 
   g.rows = g.zlo > g.zhi ? 0 : g.nby * (g.bz1 - g.bz0 + 1);
 }
 
-__global__ void k_mesh_unit_counts(MeshPatches M, Bins B, int nunits, uint32_t* __restrict__ key,
-                                   int32_t* __restrict__ unit) {
+__global__ void k_mesh_unit_counts(MeshPatches M, Bins B, int nunits, uint32_t* __restrict__ cnt,
+                                   uint32_t* __restrict__ key, int32_t* __restrict__ unit, int32_t* __restrict__ nm) {
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (u >= nunits) return;
   UnitGeo g;
   mesh_unit_geo(M, B, u, g);
-  unit_count(B, g, u, lane, key, unit);
+  unit_count(B, g, u, lane, [](int) { return 1; }, cnt, key, unit, nm);
 }
 
 // The store in bin order with each particle's weight on the level.
@@ -2551,7 +2608,8 @@ k_mesh_patch_counts(MeshPatches M, Bins B, const float4* __restrict__ P, PatchWo
   UnitGeo g;
   mesh_unit_geo(M, B, it.x, g);
   for (int q = threadIdx.x; q < MZ * NA * NA; q += blockDim.x) s_cnt[q] = 0;
-  const int64_t v0 = (int64_t)it.y * PSLICE, v1 = v0 + PSLICE;
+  const int slice = W.unit[it.x].y;
+  const int64_t v0 = (int64_t)it.y * slice, v1 = v0 + slice;
   int64_t vbase = 0;
   for (int r0 = 0; r0 < g.rows; r0 += PROWS) {
     const int nr = min(PROWS, g.rows - r0);
@@ -2575,7 +2633,7 @@ k_mesh_patch_counts(MeshPatches M, Bins B, const float4* __restrict__ P, PatchWo
     vbase += tot;
   }
   __syncthreads();
-  const bool shared = W.scratch_of[it.x] >= 0;
+  const bool shared = W.unit[it.x].x >= 0;
   const int bor = M.boramr;
   int32_t* o = out + ((size_t)g.ip * NA + g.zlo) * NA * NA;
   for (int q = threadIdx.x; q < MZ * NA * NA; q += blockDim.x) {
@@ -2591,6 +2649,7 @@ k_mesh_patch_counts(MeshPatches M, Bins B, const float4* __restrict__ P, PatchWo
 
 // Clears the output of the units that several slices share.
 __global__ void k_mesh_clear(const int32_t* __restrict__ multi, int32_t* __restrict__ out) {
+  if (multi[blockIdx.x] < 0) return;
   int32_t* o = out + (size_t)multi[blockIdx.x] * MZ * NA * NA;
   for (int q = threadIdx.x; q < MZ * NA * NA; q += blockDim.x) o[q] = 0;
 }
@@ -2651,7 +2710,7 @@ extern "C" int asohf_mesh_patch_counts(asohf_ctx* c, int nx, float lado0, float 
   const int64_t n = c->p.n;
   const size_t outb = 4 * (size_t)npatch * NA * NA * NA;
   const int nunits = MSLAB * npatch;
-  ASOHF_CHECK(arena_reserve(c, (on_device ? 0 : outb) + (24 + 4 * MSLAB) * (size_t)npatch + 16 * (size_t)n +
+  ASOHF_CHECK(arena_reserve(c, (on_device ? 0 : outb) + (24 + 8 * MSLAB) * (size_t)npatch + 16 * (size_t)n +
                                    unit_list_bytes(nunits) + bins_bytes(n, lado0, dx, 2) + 16384));
   int32_t* pn = (int32_t*)arena_alloc(c, 12 * (size_t)npatch);
   float* pr = (float*)arena_alloc(c, 12 * (size_t)npatch);
@@ -2675,8 +2734,8 @@ extern "C" int asohf_mesh_patch_counts(asohf_ctx* c, int nx, float lado0, float 
   if (n > 0)
     k_mesh_stage<<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(
         B.idx, n, c->p.x, c->p.y, c->p.z, c->rows_cur >= 0 ? c->rows[c->rows_cur] : nullptr, irpa, refine_thr, E, bp);
-  k_mesh_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, nunits, U.key, U.unit);
-  ASOHF_CHECK(unit_list_size(c, &U));
+  k_mesh_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, nunits, U.cnt, U.key, U.unit, U.nm);
+  ASOHF_CHECK(unit_list_size(c, &U, kSliceUnits));
   ASOHF_CHECK(seg_reserve(c, unit_work_bytes(U, 0)));
   PatchWork W;
   int32_t* multi;
