@@ -886,16 +886,18 @@ k_base_stencil(const int32_t* __restrict__ cnt, int nx, Terms8 T, float denbas, 
 // kernel at 384^3 with 8192, 16384, 24576 and 32768: 17.5, 16.3, 15.9, 15.7 ms),
 // small ones spread few units, or few with many wide clouds: DENSITY of 262144
 // particles on 299 patches to level 3 takes 0.38 ms with their species (0.44 with
-// slices of 24576) and 1.7 with one species (8.1); 2.1M on 2207 patches 1.43
-// (1.42) and 7.4 (10.7); 56.6M on 12012 25.6 (25.4).  Weights of 1, 8, 100 and 100
-// cut ordinary units too often (2.1M to level 6 1.82 ms, 1.77 so).
+// slices of 24576) and 1.8 with one species (8.1); 2.1M on 2207 patches 1.45
+// (1.42) and 7.4 (10.7).  Weights of 1, 8, 100 and 100 cut ordinary units too often
+// (2.1M to level 6 1.82 ms, 1.80 so).  The units still go in order of their counts:
+// in order of their work 56.6M particles took 25.7 ms, 25.3 so.
 struct SliceRule {
   int items, lo, hi;  // hi also bounds the candidates: the equal-mass kernel counts a slice's in 16 bits
   int w[4];           // weight of a cloud of level 1 or less, 2, 3, 4 or more
 };
-static const SliceRule kSliceEq{3, 8192, 24576, {1, 3, 6, 6}}, kSliceAny{6, 2048, 24576, {1, 2, 4, 13}},
+static const SliceRule kSliceEq{3, 8192, 24576, {1, 4, 6, 6}}, kSliceAny{6, 2048, 24576, {1, 2, 4, 13}},
     kSliceUnits{6, 2048, 24576, {1, 1, 1, 1}};
 #define SLICE_MIN 256  // candidates
+#define UNITS_FEW 512
 #define PROWS 128         // bin rows staged in shared memory at a time
 #define AROW (NA + 5)     // accumulator row stride (doubles): rows shifted by 5 banks pairs
 #define APLANE (NA * AROW)
@@ -944,11 +946,11 @@ __device__ __forceinline__ void row_range(const Bins& B, const UnitGeo& g, int r
   *len = b - a;
 }
 
-// Candidates of a unit (one warp per unit) and its work, candidates times their
-// weights in a sample of two a row, in sixteenths as a sort key that puts the
-// largest first.
+// Candidates of a unit (one warp per unit), as a sort key that puts the largest
+// count first, and its work: candidates times their weights in a sample of two a
+// row, in sixteenths.
 template <typename F>
-__device__ __forceinline__ void unit_count(const Bins& B, const UnitGeo& g, int u, int lane, F weight, uint32_t* cnt,
+__device__ __forceinline__ void unit_count(const Bins& B, const UnitGeo& g, int u, int lane, F weight, uint32_t* work,
                                            uint32_t* key, int32_t* unit, int32_t* nm) {
   long long s = 0, w = 0;
   for (int r = lane; r < g.rows; r += 32) {
@@ -963,8 +965,8 @@ __device__ __forceinline__ void unit_count(const Bins& B, const UnitGeo& g, int 
   }
   if (lane == 0) {
     w = (w + 15) / 16;
-    cnt[u] = (uint32_t)(s < 0xffffffffll ? s : 0xffffffffll);
-    key[u] = ~(uint32_t)(w < 0xffffffffll ? w : 0xffffffffll);
+    key[u] = ~(uint32_t)(s < 0xffffffffll ? s : 0xffffffffll);
+    work[u] = (uint32_t)(w < 0xffffffffll ? w : 0xffffffffll);
     unit[u] = u;
     if (u == 0) *nm = 0;
   }
@@ -973,7 +975,7 @@ __device__ __forceinline__ void unit_count(const Bins& B, const UnitGeo& g, int 
 // P holds the species in w, or S does (P null).
 __global__ void k_patch_unit_counts(DevMesh M, Bins B, const int32_t* __restrict__ order, int nunits, float dx,
                                     const float4* __restrict__ P, const uint8_t* __restrict__ S, SliceRule R,
-                                    uint32_t* __restrict__ cnt, uint32_t* __restrict__ key,
+                                    uint32_t* __restrict__ work, uint32_t* __restrict__ key,
                                     int32_t* __restrict__ unit, int32_t* __restrict__ nm) {
   int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (u >= nunits) return;
@@ -983,13 +985,15 @@ __global__ void k_patch_unit_counts(DevMesh M, Bins B, const int32_t* __restrict
     const int s = P ? __float_as_int(P[e].w) : (int)S[e], l = s == 255 ? 0 : g.ir - s;
     return l <= 1 ? R.w[0] : (l == 2 ? R.w[1] : (l == 3 ? R.w[2] : R.w[3]));
   };
-  unit_count(B, g, u, lane, weight, cnt, key, unit, nm);
+  unit_count(B, g, u, lane, weight, work, key, unit, nm);
 }
 
 struct PatchWork {
   const int2* items;         // (unit, slice)
   const int2* unit;          // per unit: scratch slab index (-1: one slice), candidates of a slice
   double* scratch;           // the unit's cells in float64, per multi-slice unit
+  const int* nitems;         // of a grid that may be larger, or null
+  __device__ bool past() const { return nitems && (int)blockIdx.x >= *nitems; }
 };
 
 // Rows r0 .. r0+nr-1 of a unit's bins: first entries and the running total of
@@ -1027,17 +1031,22 @@ __device__ __forceinline__ int find_row(const int* s_pre, int nr, int v) {
 }
 
 // Work items of a patch deposit, built on the device: the units in order of
-// falling work, each cut into slices.  The host reads two numbers (items, the last
-// unit with several slices) to size the buffers.  (Counts to
-// the host, sorted there and the lists sent back took 1.6 ms of the 37 ms of
-// 12012 patches at 384^3; this takes under 0.1 ms.)
+// falling candidate count, each cut into slices.  The host reads two numbers
+// (items, units with several slices) to size the buffers.  (Counts to the host,
+// sorted there and the lists sent back took 1.6 ms of the 37 ms of 12012 patches
+// at 384^3; this takes under 0.1 ms.)  Of up to UNITS_FEW units one CTA makes the
+// list in unit order, in buffers of the largest size it can take, and the host
+// reads nothing: the mesh counts of 7 patches over 32768 particles 0.21 ms, 0.25
+// with the sort, the scan and the wait.
 struct UnitList {
-  int nunits = 0, nitems = 0, nmulti = 0;
-  uint32_t* cnt = nullptr;                   // candidates, by unit
-  uint32_t *key = nullptr, *key2 = nullptr;  // ~work, by unit and sorted
+  int nunits = 0, nitems = 0, nmulti = 0;    // (bounds of the two where few)
+  bool few = false;
+  SliceRule rule{};
+  uint32_t* work = nullptr;                  // by unit
+  uint32_t *key = nullptr, *key2 = nullptr;  // ~count, by unit and sorted
   int32_t *unit = nullptr, *ord = nullptr;
   int32_t *ns = nullptr, *off = nullptr;     // slices of each sorted unit, and the sum before it
-  int32_t* nm = nullptr;                     // the last sorted unit with several, plus 1
+  int32_t *slab = nullptr, *nm = nullptr;    // scratch slab of each, and the slabs in all
   void* tmp = nullptr;
   size_t sort_b = 0, scan_b = 0;
 };
@@ -1052,63 +1061,74 @@ static void unit_list_temp(int nunits, size_t* sort_b, size_t* scan_b) {
 static size_t unit_list_bytes(int nunits) {
   size_t a, b;
   unit_list_temp(nunits, &a, &b);
-  return 36 * (size_t)nunits + (a > b ? a : b) + 16 * 256;
+  return 40 * (size_t)nunits + (a > b ? a : b) + 16 * 256;
 }
 
 static int unit_list_begin(asohf_ctx* c, int nunits, UnitList* U) {
   U->nunits = nunits;
   const size_t b = 4 * (size_t)nunits + 4;
-  U->cnt = (uint32_t*)arena_alloc(c, b);
+  U->work = (uint32_t*)arena_alloc(c, b);
   U->key = (uint32_t*)arena_alloc(c, b);
   U->key2 = (uint32_t*)arena_alloc(c, b);
   U->unit = (int32_t*)arena_alloc(c, b);
   U->ord = (int32_t*)arena_alloc(c, b);
   U->ns = (int32_t*)arena_alloc(c, b);
   U->off = (int32_t*)arena_alloc(c, b);
+  U->slab = (int32_t*)arena_alloc(c, b);
   U->nm = (int32_t*)arena_alloc(c, 4);
   unit_list_temp(nunits, &U->sort_b, &U->scan_b);
   U->tmp = arena_alloc(c, U->sort_b > U->scan_b ? U->sort_b : U->scan_b);
-  return U->cnt && U->key && U->key2 && U->unit && U->ord && U->ns && U->off && U->nm && U->tmp
+  return U->work && U->key && U->key2 && U->unit && U->ord && U->ns && U->off && U->slab && U->nm && U->tmp
              ? ASOHF_OK
              : ASOHF_ERR_CAPACITY;
 }
 
-// Slices of the sorted units (256 threads).  Every CTA forms the share of work
-// from the sum over all units: over up to 1024 of them, else over 1024 evenly
-// spaced ones (the work falls steadily) times their distance.
+// The share of work a slice holds, from that of all units (sixteenths).
+__device__ __forceinline__ double slice_share(double sum, int sms, const SliceRule& R) {
+  const double sm = 16.0 * sum / sms;  // an SM's work
+  return fmax(fmin(fmax(sm / R.items, (double)R.lo), (double)R.hi), sm / 12.0);
+}
+
+// Slices of a unit: at most 1 + work/share + cnt/hi.
+__device__ __forceinline__ int unit_slices(uint32_t cnt, uint32_t work, double share, const SliceRule& R) {
+  const double most = fmax(1.0, (double)(cnt / SLICE_MIN));
+  const int k = (int)fmin(most, ceil(16.0 * (double)work / share));
+  return max(max(k, 1), (int)((cnt + (uint64_t)R.hi - 1) / R.hi));
+}
+
+// Slices of the sorted units (256 threads).  Every CTA sums the work over up to
+// 1024 units, else over 1024 or more evenly spaced in the sorted order (the counts
+// fall steadily) times their distance.
 __global__ void k_unit_slices(const uint32_t* __restrict__ key, const int32_t* __restrict__ ord,
-                              const uint32_t* __restrict__ cnt, int n, int sms, SliceRule R, int32_t* __restrict__ ns,
-                              int32_t* __restrict__ nm) {
-  __shared__ double s_sum[8];
+                              const uint32_t* __restrict__ work, int n, int sms, SliceRule R, int32_t* __restrict__ ns,
+                              int32_t* __restrict__ slab, int32_t* __restrict__ nm) {
+  __shared__ double s_sum[32];
   const int step = n > 1024 ? n / 1024 : 1;
   double sum = 0.0;
-  for (int64_t q = (int64_t)threadIdx.x * step; q < n; q += 256 * (int64_t)step) sum += (double)(~key[q]);
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sum;
-  __syncthreads();
-  sum = 0.0;
-  for (int w = 0; w < 8; w++) sum += s_sum[w];
-  const double sm = 16.0 * sum * step / sms;  // an SM's work
-  const double share = fmax(fmin(fmax(sm / R.items, (double)R.lo), (double)R.hi), sm / 12.0);
+  for (int64_t q = (int64_t)threadIdx.x * step; q < n; q += 256 * (int64_t)step) sum += (double)work[ord[q]];
+  const double share = slice_share(block_sum_d(sum, s_sum) * step, sms, R);
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r > n) return;
-  int k = 0;
-  if (r < n) {
-    const uint32_t m = cnt[ord[r]];
-    const double most = fmax(1.0, (double)(m / SLICE_MIN));
-    k = (int)fmin(most, ceil(16.0 * (double)(~key[r]) / share));
-    k = max(max(k, 1), (int)((m + (uint64_t)R.hi - 1) / R.hi));
-  }
+  const int k = r < n ? unit_slices(~key[r], work[ord[r]], share, R) : 0;
   ns[r] = k;
-  if (k > 1) atomicMax(nm, r + 1);
+  if (r < n) slab[r] = k > 1 ? atomicAdd(nm, 1) : -1;
 }
 
 // After the counts: the sort, the slices and their sum; reads the totals.
 static int unit_list_size(asohf_ctx* c, UnitList* U, SliceRule R) {
   const int n = U->nunits;
+  const int64_t whole = c->p.n * n / R.hi;  // slices of R.hi candidates, at most
+  U->few = n <= UNITS_FEW && whole < 4096;
+  U->rule = R;
+  if (U->few) {
+    U->nitems = n + 12 * c->num_sms + (int)whole + 16;
+    U->nmulti = n;
+    return ASOHF_OK;
+  }
   ASOHF_CUDA(cub::DeviceRadixSort::SortPairs(U->tmp, U->sort_b, U->key, U->key2, U->unit, U->ord, n, 0, 32,
                                              c->stream));
-  k_unit_slices<<<n / 256 + 1, 256, 0, c->stream>>>(U->key2, U->ord, U->cnt, n, c->num_sms, R, U->ns, U->nm);
+  k_unit_slices<<<n / 256 + 1, 256, 0, c->stream>>>(U->key2, U->ord, U->work, n, c->num_sms, R, U->ns, U->slab,
+                                                     U->nm);
   ASOHF_CUDA(cub::DeviceScan::ExclusiveSum(U->tmp, U->scan_b, U->ns, U->off, n + 1, c->stream));
   c->launches++;
   int32_t h[2];
@@ -1124,20 +1144,46 @@ static size_t unit_work_bytes(const UnitList& U, int unit_cells) {
   return sizeof(int2) * (size_t)U.nitems + 4 * (size_t)U.nmulti + 8 * (size_t)unit_cells * U.nmulti + 4 * 256;
 }
 
-// multi: the unit of each scratch slab, -1 where the slab is not used.
+// multi: the unit of each scratch slab (-1: the slab is not used).
 __global__ void k_unit_items(const int32_t* __restrict__ ord, const int32_t* __restrict__ ns,
-                             const int32_t* __restrict__ off, const uint32_t* __restrict__ cnt, int n, int nmulti,
-                             int2* __restrict__ items, int2* __restrict__ unit, int32_t* __restrict__ multi) {
+                             const int32_t* __restrict__ off, const int32_t* __restrict__ slab,
+                             const uint32_t* __restrict__ key, int n, int2* __restrict__ items,
+                             int2* __restrict__ unit, int32_t* __restrict__ multi) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
-  const int u = ord[r], k = ns[r], o = off[r];
+  const int u = ord[r], k = ns[r], o = off[r], l = slab[r];
   for (int q = 0; q < k; q++) items[o + q] = make_int2(u, q);
-  unit[u] = make_int2(k > 1 ? r : -1, (int)((cnt[u] + (uint64_t)k - 1) / k));
-  if (r < nmulti) multi[r] = k > 1 ? u : -1;
+  unit[u] = make_int2(l, (int)((~key[r] + (uint64_t)k - 1) / k));
+  if (l >= 0) multi[l] = u;
+}
+
+// The list of few units, in unit order (one CTA of UNITS_FEW threads).
+__global__ void __launch_bounds__(UNITS_FEW)
+k_unit_list_few(const uint32_t* __restrict__ key, const uint32_t* __restrict__ work, int n, int sms, SliceRule R, int cap,
+                int2* __restrict__ items, int2* __restrict__ unit, int32_t* __restrict__ multi,
+                int* __restrict__ nitems) {
+  __shared__ double s_sum[32];
+  __shared__ int s_run[32];
+  const int u = threadIdx.x, lane = u & 31;
+  const double share = slice_share(block_sum_d(u < n ? (double)work[u] : 0.0, s_sum), sms, R);
+  const int k = u < n ? unit_slices(~key[u], work[u], share, R) : 0;
+  int end = k;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, end, o);
+    if (lane >= o) end += v;
+  }
+  if (lane == 31) s_run[u >> 5] = end;
+  __syncthreads();
+  for (int w = 0; w < u >> 5; w++) end += s_run[w];
+  if (u == UNITS_FEW - 1) *nitems = min(end, cap);
+  if (u >= n) return;
+  for (int q = 0; q < k && end - k + q < cap; q++) items[end - k + q] = make_int2(u, q);
+  unit[u] = make_int2(k > 1 ? u : -1, (int)((~key[u] + (uint64_t)k - 1) / k));
+  multi[u] = k > 1 ? u : -1;
 }
 
 // The items, scratch slabs (cleared) and slab indices, in buffers of the
-// caller's: `walloc` for what unit_work_bytes counts, `salloc` for 8 bytes a unit.
+// caller's: `walloc` for what unit_work_bytes counts, `salloc` for 8 bytes a unit and 8.
 template <typename FW, typename FS>
 static int unit_list_fill(asohf_ctx* c, const UnitList& U, int unit_cells, FW walloc, FS salloc, PatchWork* W,
                           int32_t** multi) {
@@ -1145,11 +1191,17 @@ static int unit_list_fill(asohf_ctx* c, const UnitList& U, int unit_cells, FW wa
   *multi = (int32_t*)walloc(4 * (size_t)(U.nmulti > 0 ? U.nmulti : 1));
   const size_t sb = 8 * (size_t)unit_cells * U.nmulti;
   W->scratch = (double*)walloc(sb > 0 ? sb : 8);
-  int2* unit = (int2*)salloc(8 * (size_t)U.nunits);
+  int2* unit = (int2*)salloc(8 * (size_t)U.nunits + 8);
+  int* nitems = (int*)(unit + U.nunits);
   if (!items || !*multi || !W->scratch || !unit) return ASOHF_ERR_CAPACITY;
   if (sb) ASOHF_CUDA(cudaMemsetAsync(W->scratch, 0, sb, c->stream));
-  k_unit_items<<<(U.nunits + 255) / 256, 256, 0, c->stream>>>(U.ord, U.ns, U.off, U.cnt, U.nunits, U.nmulti, items,
-                                                                   unit, *multi);
+  W->nitems = U.few ? nitems : nullptr;
+  if (U.few)
+    k_unit_list_few<<<1, UNITS_FEW, 0, c->stream>>>(U.key, U.work, U.nunits, c->num_sms, U.rule, U.nitems, items, unit,
+                                                    *multi, nitems);
+  else
+    k_unit_items<<<(U.nunits + 255) / 256, 256, 0, c->stream>>>(U.ord, U.ns, U.off, U.slab, U.key2, U.nunits, items,
+                                                                unit, *multi);
   c->launches++;
   W->items = items;
   W->unit = unit;
@@ -1228,6 +1280,7 @@ k_density_patches_eq(DevMesh M, Bins B, const float4* __restrict__ P, const int3
   __shared__ unsigned short s_l2[LCAP], s_l2s[LCAP + 1];  // listed level-2 clouds, and sorted
   __shared__ int s_nl2, s_off2[NB2 + 1], s_cur2[NB2];
   const unsigned FULL = 0xffffffffu;
+  if (W.past()) return;
   const int2 it = W.items[blockIdx.x];
   UnitGeo g;
   unit_geo(M, B, order, it.x, dx, g);
@@ -1509,6 +1562,7 @@ k_density_patches(DevMesh M, Bins B, const float4* __restrict__ P, const uint8_t
                   float* __restrict__ u11, const float* __restrict__ denbas_lev) {
   extern __shared__ double acc[];  // ACC_N doubles (padded rows), kernel table
   float* ktab = (float*)(acc + ACC_N);
+  if (W.past()) return;
   const int2 it = W.items[blockIdx.x];
   __shared__ int s_lo[PROWS], s_pre[PROWS + 1], s_next;
   __shared__ float s_rcp[NA + 1];  // 1/n for the clipped cloud widths n <= NA
@@ -1868,7 +1922,7 @@ extern "C" int asohf_density(asohf_ctx* c, int nx, float lado0, float dx, float 
       ASOHF_CHECK(unit_list_begin(c, nunits, &U));
       const SliceRule R = pd_eq ? kSliceEq : kSliceAny;
       k_patch_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, order, nunits, dx, pd_eq ? bp : nullptr, bs, R,
-                                                                   U.cnt, U.key, U.unit, U.nm);
+                                                                   U.work, U.key, U.unit, U.nm);
       c->launches++;
       // work list: slices of the candidates, the densest units first; in
       // the segment buffers, or density pool 1 when deferred
@@ -2249,6 +2303,7 @@ k_tsc_patches(DevMesh M, Bins B, const float4* __restrict__ P, PatchWork W, floa
   __shared__ float s_w[TSC_BLOCK / 32][32 * TSC_WARP_W];
   __shared__ int s_lo[PROWS], s_pre[PROWS + 1], s_next;
   const unsigned FULL = 0xffffffffu;
+  if (W.past()) return;
   const int2 it = W.items[blockIdx.x];
   UnitGeo g;
   tsc_unit_geo(M, B, it.x, dx, g);
@@ -2329,13 +2384,13 @@ k_tsc_patches(DevMesh M, Bins B, const float4* __restrict__ P, PatchWork W, floa
   }
 }
 
-__global__ void k_tsc_unit_counts(DevMesh M, Bins B, int nunits, float dx, uint32_t* __restrict__ cnt,
+__global__ void k_tsc_unit_counts(DevMesh M, Bins B, int nunits, float dx, uint32_t* __restrict__ work,
                                   uint32_t* __restrict__ key, int32_t* __restrict__ unit, int32_t* __restrict__ nm) {
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (u >= nunits) return;
   UnitGeo g;
   tsc_unit_geo(M, B, u, dx, g);
-  unit_count(B, g, u, lane, [](int) { return 1; }, cnt, key, unit, nm);
+  unit_count(B, g, u, lane, [](int) { return 1; }, work, key, unit, nm);
 }
 
 // Units shared by several slices: the summed scratch slab to U11.
@@ -2428,7 +2483,7 @@ extern "C" int asohf_interpolate_density_tsc(asohf_ctx* c, int nx, float lado0, 
       if (!dden) return ASOHF_ERR_CAPACITY;
       UnitList U;
       ASOHF_CHECK(unit_list_begin(c, nunits, &U));
-      k_tsc_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, nunits, dx, U.cnt, U.key, U.unit, U.nm);
+      k_tsc_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, nunits, dx, U.work, U.key, U.unit, U.nm);
       c->launches++;
       ASOHF_CHECK(unit_list_size(c, &U, kSliceUnits));
       ASOHF_CHECK(seg_reserve(c, unit_work_bytes(U, NA * NA * TZ)));
@@ -2578,13 +2633,13 @@ __device__ __forceinline__ void mesh_unit_geo(const MeshPatches& M, const Bins& 
   g.rows = g.zlo > g.zhi ? 0 : g.nby * (g.bz1 - g.bz0 + 1);
 }
 
-__global__ void k_mesh_unit_counts(MeshPatches M, Bins B, int nunits, uint32_t* __restrict__ cnt,
+__global__ void k_mesh_unit_counts(MeshPatches M, Bins B, int nunits, uint32_t* __restrict__ work,
                                    uint32_t* __restrict__ key, int32_t* __restrict__ unit, int32_t* __restrict__ nm) {
   const int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (u >= nunits) return;
   UnitGeo g;
   mesh_unit_geo(M, B, u, g);
-  unit_count(B, g, u, lane, [](int) { return 1; }, cnt, key, unit, nm);
+  unit_count(B, g, u, lane, [](int) { return 1; }, work, key, unit, nm);
 }
 
 // The store in bin order with each particle's weight on the level.
@@ -2604,6 +2659,7 @@ __global__ void __launch_bounds__(256)
 k_mesh_patch_counts(MeshPatches M, Bins B, const float4* __restrict__ P, PatchWork W, int32_t* __restrict__ out) {
   __shared__ int32_t s_cnt[MZ * NA * NA];
   __shared__ int s_lo[PROWS], s_pre[PROWS + 1];
+  if (W.past()) return;
   const int2 it = W.items[blockIdx.x];
   UnitGeo g;
   mesh_unit_geo(M, B, it.x, g);
@@ -2734,7 +2790,7 @@ extern "C" int asohf_mesh_patch_counts(asohf_ctx* c, int nx, float lado0, float 
   if (n > 0)
     k_mesh_stage<<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(
         B.idx, n, c->p.x, c->p.y, c->p.z, c->rows_cur >= 0 ? c->rows[c->rows_cur] : nullptr, irpa, refine_thr, E, bp);
-  k_mesh_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, nunits, U.cnt, U.key, U.unit, U.nm);
+  k_mesh_unit_counts<<<(nunits + 7) / 8, 256, 0, c->stream>>>(M, B, nunits, U.work, U.key, U.unit, U.nm);
   ASOHF_CHECK(unit_list_size(c, &U, kSliceUnits));
   ASOHF_CHECK(seg_reserve(c, unit_work_bytes(U, 0)));
   PatchWork W;

@@ -1,5 +1,5 @@
 """Work lists whose slices are the smallest, the largest and in between (their
-size follows the candidates of a call): 1 to 40 patches over one crowded core,
+size follows the work of a call): 1 to 130 patches over one crowded core,
 in the patch deposits of one and of several masses, in the TSC and in the mesh
 counts.  The deposits sum the same REAL*4 terms in float64 as the oracle and
 round once: equal but at a rounding boundary, one float32 spacing; the counts
@@ -34,7 +34,9 @@ def patches(k, dx):
     return synth.Mesh(1, np.array([0, k], np.int32), *size, *(corner + 1), *pr, np.zeros(k, np.int32))
 
 
-CASES = [(600, 1), (9000, 1), (9000, 5), (120000, 12), (200000, 40)]
+# units of up to 512 (64 patches of 8, 128 of 4) and few enough slices: the list of one CTA, else the sorted one
+CASES = [(600, 1), (9000, 1), (9000, 5), (120000, 12), (200000, 40), (3000, 64), (3000, 65), (200000, 64), (2000, 128),
+         (2000, 129), (60000, 130)]
 
 
 @pytest.mark.parametrize("n,k", CASES)
