@@ -132,8 +132,9 @@ class Asohf:
         _check(self.L.asohf_set_epot_seed(self.h, C.c_uint32(int(seed))), "asohf_set_epot_seed")
 
     def set_cluster_threshold(self, min_members: int):
-        """Haloes with at least min_members members go to the cluster path
-        (0: default)."""
+        """Haloes with at least min_members members go to the cluster path (0: by
+        the call's members, not below tier 2), subhaloes from the smaller of it
+        and max(tier 2, 2048) members on."""
         _check(self.L.asohf_set_cluster_threshold(self.h, C.c_int64(int(min_members))),
                "asohf_set_cluster_threshold")
 

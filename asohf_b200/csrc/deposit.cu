@@ -760,12 +760,10 @@ static int upload_mesh(asohf_ctx* c, const asohf_mesh* mh, DevMesh* d, DAlloc A 
 }
 
 // ------------------------------------------------------------ staging
-// The store in bin order as float4 (x, y, z, m) plus the species index (in
-// the mass's place when all masses are equal), so a patch reads its candidates as contiguous runs (one run per (y, z) row of
-// bins).
+// The store in bin order as float4 (x, y, z, m) plus the species index (in the
+// mass's place when all masses are equal), so a patch reads its candidates as
+// contiguous runs (one run per (y, z) row of bins).
 #define NA ASOHF_NAMRX
-#define ZH (NA / 2)
-#define PD_BLOCK 512
 
 __global__ void k_bin_stage(const int32_t* __restrict__ idx, int64_t n, int64_t ndep, const float* __restrict__ x,
                             const float* __restrict__ y, const float* __restrict__ z, const float* __restrict__ m,

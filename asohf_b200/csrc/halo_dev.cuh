@@ -452,11 +452,6 @@ __device__ __forceinline__ void query_box_w(const ColIdx& ci, float cx, float cy
   }
 }
 
-template <class F>
-__device__ __forceinline__ void query_box(const ColIdx& ci, float cx, float cy, float cz, float r, F&& f) {
-  query_box_w(ci, cx, cy, cz, r, threadIdx.x >> 5, blockDim.x >> 5, f);
-}
-
 // Group query balanced by entries: every CTA finds the x ranges of all the
 // query's columns (up to QMAX) into shared memory, then the group's warps
 // take equal contiguous shares of the concatenated ranges, so a few dense

@@ -95,8 +95,10 @@ int asohf_set_epot_seed(asohf_ctx *ctx, uint32_t seed);
 /* Tuning, no counterpart in the reference: haloes with at least
  * min_members members are refined by a thread-block cluster, the others by
  * one CTA each (results are the same either way).  0 restores the default
- * (1/256 of the members a call counts, between 2048 and 32768); 1 sends every
- * halo to the cluster path. */
+ * (1/256 of the members a call counts, between 2048 and 32768 and not below
+ * tier2_members); 1 sends every halo to the cluster path.  The subhalo call
+ * takes clusters from the smaller of min_members and max(tier2_members, 2048)
+ * members on. */
 int asohf_set_cluster_threshold(asohf_ctx *ctx, int64_t min_members);
 /* Tuning, no counterpart in the reference: the halo kernel gives a
  * cluster-tier halo 16 CTAs above 8 x members_per_cta members, 8 above
