@@ -488,6 +488,7 @@ int level_runs(asohf_ctx* c, const asohf_catalogue* cat, int n, int on_device, s
     if (n) ASOHF_CUDA(cudaMemcpyAsync(lev, cat->levhal, 4 * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
     ASOHF_CUDA(cudaStreamSynchronize(c->stream));
   } else if (n) {
+    if (!cat->levhal) return ASOHF_ERR_INVALID;
     memcpy(lev, cat->levhal, 4 * (size_t)n);
   }
   for (int i = 1; i < n; i++)

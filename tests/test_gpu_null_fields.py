@@ -11,7 +11,7 @@ from asohf_b200 import abi, api, driver, synth
 pytestmark = pytest.mark.gpu
 INVALID = 1
 PRUNE = ["clusrx", "radio", "realclus", "dmpclus"]
-CLEAN = ["clusry", "vx", "masa", "realclus"]
+CLEAN = ["clusry", "vx", "masa", "levhal", "realclus"]
 OVERLAP = ["clusrz", "radio", "levhal", "realclus"]
 ALL = ["clusrx", "masa", "vcmax", "dmpclus", "iplip", "profiles", "inertia_tensor", "indcs"]
 
