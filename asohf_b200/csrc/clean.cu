@@ -615,7 +615,8 @@ extern "C" int asohf_overlapping(asohf_ctx* c, asohf_catalogue* cat, int ir, con
   const float pi = (float)acos(-1.0);
   const OverlapGeo g{pi / 12.0f, 4.0f * pi / 3.0f, vol_solap_low};
   const int nw = (n + 31) >> 5;
-  const bool smem = (size_t)nw * 4 <= 192u * 1024u;
+  const size_t most = 192u * 1024u;  // dynamic shared memory of the replay
+  const bool smem = (size_t)nw * 4 <= most;
   int cap = 2 * n + 1024, cnt[2] = {0, 0};
   unsigned long long *keys = nullptr, *keys2 = nullptr;
   uint32_t* gbits = nullptr;
@@ -649,7 +650,9 @@ extern "C" int asohf_overlapping(asohf_ctx* c, asohf_catalogue* cat, int ir, con
       c->launches++;
     }
   const size_t dyn = smem ? 4 * (size_t)nw : 0;
-  ASOHF_CUDA(cudaFuncSetAttribute(k_overlap_replay, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+  // the limit belongs to the process: the same for every call, so that no other
+  // thread's lowers it before this launch
+  ASOHF_CUDA(cudaFuncSetAttribute(k_overlap_replay, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   k_overlap_replay<<<1, 1024, dyn, c->stream>>>(io.d.rc, n, j0, j1, keys2, cap, dw, b, gbits, smem ? 1 : 0,
                                                 dw + 4);
   c->launches++;

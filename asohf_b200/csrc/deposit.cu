@@ -1932,10 +1932,14 @@ extern "C" int asohf_density(asohf_ctx* c, int nx, float lado0, float dx, float 
       ASOHF_CHECK(unit_list_fill(c, U, NA * NA * PZ,
                                  [&](size_t b) { return defer ? dpool_alloc(c, 1, b) : seg_alloc(c, b); },
                                  [&](size_t b) { return A.get(b); }, &W, &dmulti));
-      const size_t smem = (pd_eq ? sizeof(uint32_t) * CGP * CG * CG + sizeof(float) * 4 * T2COPY
-                                 : sizeof(double) * ACC_N) + sizeof(float) * ktab_size(nl);
+      const size_t smem0 = pd_eq ? sizeof(uint32_t) * CGP * CG * CG + sizeof(float) * 4 * T2COPY
+                                 : sizeof(double) * ACC_N;
+      const size_t smem = smem0 + sizeof(float) * ktab_size(nl);
+      // the limit belongs to the process: the same whatever the levels of a call,
+      // so that no other thread's call lowers it before this launch
       ASOHF_CUDA(cudaFuncSetAttribute(pd_eq ? (const void*)k_density_patches_eq : (const void*)k_density_patches,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(smem0 + sizeof(float) * ktab_size(ASOHF_NLEVELS))));
       // deferred: the patch kernels run on the density stream after the
       // staging above, and the call returns without waiting for them
       cudaStream_t ps = c->stream;
